@@ -17,7 +17,7 @@ __device__ __forceinline__ void h_coeffs(T a, T chx, T chy, T& fh, T& cx, T& cy)
     const T den = T(1) + a;
     fh = (T(1) - a) / den;
     cx = chx / den;
-    cy = chy / den;
+    cy = chy == chx ? cx : chy / den;  // square cells: the same quotient
   }
 }
 

@@ -19,6 +19,8 @@
 //
 // After the tile is written, the block applies the source and monitor
 // operations that fall inside it, spread over all its threads.
+#include <atomic>
+
 #include "bz_stencil.cuh"
 
 namespace bz {
@@ -31,7 +33,7 @@ template <typename T>
 struct Geo2D {
   int nx, ny, pitch, n_designs, n_mat;
   long long plane;  // ny * pitch
-  T chx, chy, qy, inv_kd2;
+  T chx, chy, qy, inv_kd2, one;  // one = 1, kept out of the compiler's sight
 };
 
 template <typename T>
@@ -258,220 +260,415 @@ __global__ void __launch_bounds__(BX) step2d_kernel(
 
 // ---- temporal blocking ---------------------------------------------------------
 // step2d_tb_kernel advances TS (odd) steps per launch. A block holds a tile of 64
-// columns x NW*R rows in registers: lane l of warp w owns columns X0+l and X0+32+l
-// (coalesced loads) of rows Y0+w*R .. Y0+w*R+R-1, together with their update
-// factors. Each sub-step is the single-step update restricted to the tile; the
-// values next to the tile's edges go stale by one cell per sub-step, so after TS
-// sub-steps the tile minus TS cells on every side (the owned box, which tiles the
-// grid) is exact, and only it is stored. x neighbours come from shuffles, the rows
-// across warps from shared memory (two barriers per sub-step). Sources act on every
-// tile cell (halo cells have to evolve like the real ones); monitors sample owned
-// cells only. Reads copy (step & 1) and writes the other, like TS single steps.
-template <typename T, int NC, int TS, int R, int NW>
-__global__ void __launch_bounds__(32 * NW) step2d_tb_kernel(
+// columns x NW*R rows in registers: lane l of warp w owns columns X0+2l, X0+2l+1 of
+// rows Y0+w*R .. Y0+w*R+R-1. Each sub-step is the single-step update restricted to
+// the tile; the values next to the tile's edges go stale by one cell per sub-step, so
+// after TS sub-steps the tile minus a halo (TS+1 columns, TS rows a side) is exact, and
+// only it is stored. Reads copy (step & 1) and writes the other, like TS single steps.
+//
+// What bounds it is issue and latency, not memory (the grid stays in L2 for TS steps):
+//  * The two columns of a lane are one packed operand (add/mul/fma.f32x2: the same
+//    rounding per element), one shuffle a row and field moves the x neighbour.
+//  * A tile without loss and off the grid's edge (most tiles) needs no factor but ce
+//    (fh = fe = 1 exactly), so a cell costs four registers and two blocks share an SM:
+//    one loads while the other computes. Other tiles keep fh, cx, cy and fe in shared
+//    memory.
+//  * One block barrier a sub-step: a warp receives Ez of the rows above and below it
+//    and carries the new Hy of the row above itself (one redundant row of updates).
+//  * Every lane looks up its own cells' operations (a shared-memory map filled once per
+//    launch), so the points of a line along x are handled by the lanes in parallel.
+// Components of a complex field are independent real fields (real coefficients) and
+// run as separate blocks.
+//
+// Measured against the same tile with five factors a cell in registers, two barriers a
+// sub-step and the operations walked one by one (us a launch, before -> after): 2000 x
+// 1000 cells with a line source and three lines of points, 7 steps, 57.5 -> 35.0; 400 x
+// 400 with four recorded edge lines, 9 steps, 49.3 -> 16.5; two components of 1000 x 501,
+// 7 steps, 34.9 -> 26.7; 64 designs of 600 x 400, 7 steps, 481 -> 297; float64 601 x 397,
+// 9 steps, 32.9 -> 25.1. A sub-step of two co-resident tiles clear of loss takes about
+// 900 cycles, of which the packed arithmetic fills about 730; the tile's loads take 3000
+// to 6000 cycles a launch. Measured slower: all shuffles of a pass ahead of its
+// arithmetic (1070 cycles; more registers live), x differences as single subtractions
+// instead of packed ones (1150).
+constexpr int TBW = 64;  // tile columns
+
+// Pairs of neighbouring cells: float pairs stay packed in one 64-bit register through the
+// whole launch (unpacking and packing again would cost more than the arithmetic).
+typedef unsigned long long f32pair;
+template <typename T>
+struct PairOf;
+template <>
+struct PairOf<float> {
+  typedef f32pair type;
+};
+template <>
+struct PairOf<double> {
+  typedef double2 type;
+};
+
+__device__ __forceinline__ f32pair mk2(float a, float b) {
+  f32pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float lo2(f32pair v) {
+  return __uint_as_float((unsigned)v);
+}
+__device__ __forceinline__ float hi2(f32pair v) {
+  return __uint_as_float((unsigned)(v >> 32));
+}
+__device__ __forceinline__ f32pair mul2(f32pair a, f32pair b) {
+  f32pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32pair fma2(f32pair a, f32pair b, f32pair c) {
+  f32pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a - b as one fused multiply-add with -1: a single rounding, as the subtraction's
+__device__ __forceinline__ f32pair sub2(f32pair a, f32pair b) { return fma2(b, mk2(-1.f, -1.f), a); }
+__device__ __forceinline__ bool nonzero2(f32pair v) { return v != 0ull; }
+
+__device__ __forceinline__ double2 mk2(double a, double b) { return make_double2(a, b); }
+__device__ __forceinline__ double lo2(double2 v) { return v.x; }
+__device__ __forceinline__ double hi2(double2 v) { return v.y; }
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)); }
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
+  return make_double2(__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y));
+}
+__device__ __forceinline__ double2 sub2(double2 a, double2 b) { return make_double2(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)); }
+__device__ __forceinline__ bool nonzero2(double2 v) { return v.x != 0.0 || v.y != 0.0; }
+
+template <typename T>
+__device__ __forceinline__ typename PairOf<T>::type ldg2(const T* p) {
+  return __ldg(reinterpret_cast<const typename PairOf<T>::type*>(p));
+}
+// The same with the cells that exist (e0, e1) and arrays that may be aligned to T only.
+template <typename T>
+__device__ __forceinline__ typename PairOf<T>::type ld_pair(const T* p, bool e0, bool e1) {
+  return mk2(e0 ? __ldg(p) : T(0), e1 ? __ldg(p + 1) : T(0));
+}
+
+template <typename T>
+__device__ __forceinline__ void put3(T* p, T a, T b, T c) {
+  p[0] = a;
+  p[1] = b;
+  p[2] = c;
+}
+template <typename T>
+__device__ __forceinline__ void put5(T* p, T a, T b, T c, T d, T e) {
+  p[0] = a;
+  p[1] = b;
+  p[2] = c;
+  p[3] = d;
+  p[4] = e;
+}
+
+// Shared memory of a block: factors of the tiles that need them, the rows exchanged
+// between warps (two buffers), per cell the operation on it, and the operations' values.
+constexpr int TB_POOL = 160;  // source operations of a tile held on chip; further ones are read from memory
+constexpr int TB_REC = 256;     // pairs of cells staged for monitor points each sub-step
+constexpr int TB_POINTS = 256;  // monitor points of a tile written from the staged cells
+template <typename T, int TS, int R, int NW>
+struct TbSmem {
+  static constexpr int TH = NW * R;
+  static constexpr int FAC = 4 * TH * TBW * (int)sizeof(T);
+  static constexpr int EXCH = 2 * 2 * NW * TBW * (int)sizeof(T);
+  static constexpr int POOL = (TS + 1) * TB_POOL * (int)sizeof(T);
+  static constexpr int MAP = TH * TBW * (int)sizeof(short);
+  static constexpr int REC = 2 * TB_REC * 10 * (int)sizeof(T);
+  static constexpr int LIST = 2 * TB_POINTS * (int)sizeof(int);
+  static constexpr int BYTES = FAC + EXCH + POOL + REC + LIST + MAP + 16;
+};
+
+// The operations of this warp's rows are one range of the sorted list; the lanes read it
+// side by side (row by row, or by searching, would chain dependent loads). Calls
+// f(row, column, k, single) for the first operation of each cell in columns [c0, c1) of
+// the tile; single: no other operation on the cell. Returns the rows that have any.
+template <typename F>
+__device__ __forceinline__ unsigned scan_ops(const int* __restrict__ cells, int k0, int k1, int nx, int yb, int X0,
+                                             int c0, int c1, int lane, F f) {
+  unsigned rows = 0u;
+  for (int k = k0 + lane; k < k1; k += 32) {
+    const int c = __ldg(cells + k), prev = k > k0 ? __ldg(cells + k - 1) : -1, next = k + 1 < k1 ? __ldg(cells + k + 1) : -1;
+    const int y = c / nx, x = c - y * nx;
+    if (c == prev || x < c0 || x >= c1) continue;
+    f(y - yb, x - X0, k, c != next);
+    rows |= 1u << (y - yb);
+  }
+  return __reduce_or_sync(FULL, rows);
+}
+
+template <typename T, int TS, int R, int NW, int MINB>
+__global__ void __launch_bounds__(32 * NW, MINB) step2d_tb_kernel(
     const T* __restrict__ ez_in, const T* __restrict__ hx_in, const T* __restrict__ hy_in,
     T* __restrict__ ez_out, T* __restrict__ hx_out, T* __restrict__ hy_out,
-    const T* __restrict__ ce, const T* __restrict__ loss, Geo2D<T> g, Ops2D<T> o, long long step_base,
-    const long long* __restrict__ d_step) {
-  constexpr int TW = 64, TH = NW * R;
-  constexpr int OW = TW - 2 * TS, OH = TH - 2 * TS;
-  static_assert(TS % 2 == 1 && OH > 0 && R * 2 <= 32, "bad temporal tile");
+    const T* __restrict__ ce, const T* __restrict__ loss, Geo2D<T> g, Ops2D<T> o, int n_comp, int plane0,
+    int n_planes, bool vec, long long step_base, const long long* __restrict__ d_step) {
+  typedef typename PairOf<T>::type V;
+  typedef TbSmem<T, TS, R, NW> S;
+  constexpr int TH = S::TH, HX = TS + 1;
+  constexpr int OW = TBW - 2 * HX, OH = TH - 2 * TS;
+  static_assert(TS % 2 == 1 && OW > 0 && OH > 0 && R <= 16, "bad temporal tile");
+  extern __shared__ __align__(16) unsigned char tb_smem[];
+  V* s_fac = reinterpret_cast<V*>(tb_smem);                              // [4][TH][32]: fh, -cx, cy, fe
+  V* s_ex = reinterpret_cast<V*>(tb_smem + S::FAC);                      // [2][2][NW][32]: first, last rows' Ez
+  T* s_pool = reinterpret_cast<T*>(tb_smem + S::FAC + S::EXCH);          // [TS + 1][TB_POOL]: addends, factor
+  T* s_rec = s_pool + (TS + 1) * TB_POOL;                                // [2][TB_REC][10]: staged cells
+  int2* s_list = reinterpret_cast<int2*>(tb_smem + S::FAC + S::EXCH + S::POOL + S::REC);  // (staged cell, point)
+  int* s_used = reinterpret_cast<int*>(s_list + TB_POINTS);              // slots taken: sources, points, staged cells
+  short* s_map = reinterpret_cast<short*>(s_used + 4);                   // [TH][64]: sources
+
   const long long step0 = d_step ? (__ldg(d_step) + step_base) : step_base;
   const int nx = g.nx, ny = g.ny, pitch = g.pitch;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int d = blockIdx.z;
-  const int X0 = (int)blockIdx.x * OW - TS, Y0 = (int)blockIdx.y * OH - TS;
-  const int yb = Y0 + w * R;
-  const long long fb = (long long)d * NC * g.plane;
-  const long long mb = (g.n_mat > 1 ? (long long)d : 0LL) * g.plane;
+  const int dc = plane0 + blockIdx.z, d = dc / n_comp, comp = dc - d * n_comp;  // one component per block
+  const int X0 = (int)blockIdx.x * OW - HX, Y0 = (int)blockIdx.y * OH - TS;
+  const int yb = Y0 + w * R, xa = X0 + 2 * lane, tr0 = w * R;
+  const long long fb = (long long)dc * g.plane + (long long)yb * pitch + xa;  // the thread's first cell
+  const long long mb = (g.n_mat > 1 ? (long long)d : 0LL) * g.plane + (long long)yb * pitch + xa;
+  // tiles whose every cell is an interior one of the grid skip all bounds
+  const bool inner = X0 >= 1 && X0 + TBW - 1 <= nx - 2 && Y0 >= 1 && Y0 + TH - 1 <= ny - 2;
 
-  __shared__ T s_top[NW][NC][TW];  // first row's Ez of each warp, before the H update
-  __shared__ T s_bot[NW][NC][TW];  // last row's new Hy of each warp
-  __shared__ int s_src[TH][2], s_mon[TH][2];  // op ranges of each tile row
+  // the operations' list ranges first: their latency overlaps the tile's loads
+  int sk0 = 0, sk1 = 0, mk0 = 0, mk1 = 0;
+  const int mlo = max(Y0 + TS, max(yb, 0)), mhi = min(min(Y0 + TH - TS, ny), yb + R);
+  if (o.n_src > 0 && max(yb, 0) < min(yb + R, ny)) {
+    sk0 = __ldg(o.src_row + max(yb, 0));
+    sk1 = __ldg(o.src_row + min(yb + R, ny));
+  }
+  if (o.n_mon > 0 && mlo < mhi) {
+    mk0 = __ldg(o.mon_row + mlo);
+    mk1 = __ldg(o.mon_row + mhi);
+  }
+  if (threadIdx.x < 3) s_used[threadIdx.x] = 0;
 
-  // row pointers of the op lists first, so their latency overlaps the tile loads
-  int rs_lo = 0, rs_hi = 0, rm_lo = 0, rm_hi = 0;
-  if (lane < R) {
-    const int y = yb + lane;
-    if (y >= 0 && y < ny) {
-      if (o.n_src > 0) {
-        rs_lo = __ldg(o.src_row + y);
-        rs_hi = __ldg(o.src_row + y + 1);
-      }
-      if (o.n_mon > 0) {
-        rm_lo = __ldg(o.mon_row + y);
-        rm_hi = __ldg(o.mon_row + y + 1);
-      }
-    }
-  }
-
-  int xs[2];
-  xs[0] = X0 + lane;
-  xs[1] = X0 + 32 + lane;
-  T ez[R][2][NC], hx[R][2][NC], hy[R][2][NC];
-  // Cells whose H or E the reference never changes (Hx in the last column, Hy in the
-  // last row, E on the PEC ring, everything outside the grid) get factors that keep
-  // the value: cx = 0 / cy = 0 for H (those values start and stay zero), fe = 1 and
-  // ce = 0 for E. The sub-step loop then needs no per-cell masks.
-  T fh[R][2], cx[R][2], cy[R][2], fe[R][2], cc[R][2];
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int y = yb + i;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int x = xs[j];
-      const bool in = x >= 0 && x < nx && y >= 0 && y < ny;
-      const long long r = in ? (long long)y * pitch + x : 0LL;
-      const T a = in ? __ldg(loss + mb + r) : T(0);
-      const T c = in ? __ldg(ce + mb + r) : T(0);
-      h_coeffs(a, g.chx, g.chy, fh[i][j], cx[i][j], cy[i][j]);
-      const bool interior = x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2;
-      fe[i][j] = interior ? sub_rn(T(1), mul_rn(mul_rn(a, c), g.inv_kd2)) : T(1);
-      cc[i][j] = interior ? c : T(0);
-      if (!(in && x < nx - 1)) cx[i][j] = T(0);
-      if (!(in && y < ny - 1)) cy[i][j] = T(0);
-#pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        const long long off = fb + k * g.plane + r;
-        ez[i][j][k] = in ? __ldg(ez_in + off) : T(0);
-        hx[i][j][k] = (in && x < nx - 1) ? __ldg(hx_in + off) : T(0);
-        hy[i][j][k] = (in && y < ny - 1) ? __ldg(hy_in + off) : T(0);
-      }
-    }
-  }
-  // Operation ranges: sources over the tile's columns, monitors over the owned ones.
-  if (lane < R) {
-    const int y = yb + lane, tr = w * R + lane;
-    int s0 = 0, s1 = 0, m0 = 0, m1 = 0;
-    if (y >= 0 && y < ny) {
-      if (o.n_src > 0) {
-        const int lo = rs_lo, hi = rs_hi;
-        if (lo < hi) {
-          s0 = lower_bound_i(o.src_cell, lo, hi, y * nx + max(X0, 0));
-          s1 = lower_bound_i(o.src_cell, s0, hi, y * nx + min(X0 + TW, nx));
-        }
-      }
-      if (o.n_mon > 0 && tr >= TS && tr < TH - TS) {
-        const int lo = rm_lo, hi = rm_hi;
-        if (lo < hi) {
-          m0 = lower_bound_i(o.mon_cell, lo, hi, y * nx + X0 + TS);
-          m1 = lower_bound_i(o.mon_cell, m0, hi, y * nx + min(X0 + TW - TS, nx));
-        }
-      }
-    }
-    s_src[tr][0] = s0;
-    s_src[tr][1] = s1;
-    s_mon[tr][0] = m0;
-    s_mon[tr][1] = m1;
-  }
-  __syncwarp();
-  unsigned src_rows = 0u, mon_rows = 0u;
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    if (s_src[w * R + i][0] < s_src[w * R + i][1]) src_rows |= 1u << i;
-    if (s_mon[w * R + i][0] < s_mon[w * R + i][1]) mon_rows |= 1u << i;
-  }
-  bool own[2];
-  own[0] = lane >= TS && xs[0] < nx;
-  own[1] = lane < 32 - TS && xs[1] < nx;
-  // owned cells inside the capture box (adjoint recompute): bit i*2+j
-  unsigned cap = 0u;
-  if (o.region != nullptr) {
+  V ez[R], hx[R], hy[R], cc[R], ls[R];
+  V hyu;  // Hy of the row above the warp's first; stale, as all halo rows, for warp 0
+  if (inner && vec) {
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const int tr = w * R + i, y = yb + i;
+      const int r = i * pitch;
+      ls[i] = ldg2(loss + mb + r);
+      ez[i] = ldg2(ez_in + fb + r);
+      hx[i] = ldg2(hx_in + fb + r);
+      hy[i] = ldg2(hy_in + fb + r);
+      cc[i] = ldg2(ce + mb + r);
+    }
+    hyu = ldg2(hy_in + fb - pitch);  // inside the grid also for warp 0, whose copy is never used as exact
+  } else {
+    const bool in0 = xa >= 0 && xa < nx, in1 = xa >= 0 && xa + 1 < nx;
+    const bool inm0 = in0 && xa < nx - 1, inm1 = in1 && xa + 1 < nx - 1;  // columns of Hx
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int rx = xs[j] - o.rx0, ry = y - o.ry0;
-        if (own[j] && tr >= TS && tr < TH - TS && y < ny && rx >= 0 && rx < o.rw && ry >= 0 && ry < o.rh)
-          cap |= 1u << (i * 2 + j);
+    for (int i = 0; i < R; ++i) {
+      const int y = yb + i, r = i * pitch;
+      const bool iny = y >= 0 && y < ny, inh = y >= 0 && y < ny - 1;
+      ls[i] = ld_pair(loss + mb + r, in0 && iny, in1 && iny);
+      ez[i] = ld_pair(ez_in + fb + r, in0 && iny, in1 && iny);
+      hx[i] = ld_pair(hx_in + fb + r, inm0 && iny, inm1 && iny);
+      hy[i] = ld_pair(hy_in + fb + r, in0 && inh, in1 && inh);
+      cc[i] = ld_pair(ce + mb + r, in0 && iny, in1 && iny);
+    }
+    hyu = ld_pair(hy_in + fb - pitch, in0 && yb >= 1 && yb < ny, in1 && yb >= 1 && yb < ny);
+  }
+  __syncthreads();  // the pools' counters are set
+
+  // Sources act on every tile cell (halo cells evolve like the real ones). A cell's map
+  // entry is the pool slot of its only operation, -1 for none, -2 - n for several (or no
+  // slot left), found from the warp's n-th list entry on.
+  unsigned src_rows = 0u, mon_rows = 0u, mon_lanes = 0u;
+  bool src_many = false, mon_staged = false, mon_direct = false;
+  int rec0 = 0;  // the warp's first staged pair
+  short* const w_src = s_map + tr0 * TBW;
+  if (sk0 < sk1) {
+    for (int i = lane; i < R * TBW; i += 32) w_src[i] = -1;
+    __syncwarp();
+    src_rows = scan_ops(o.src_cell, sk0, sk1, nx, yb, X0, max(X0, 0), min(X0 + TBW, nx), lane,
+                        [&](int i, int col, int k, bool single) {
+      int slot = single ? atomicAdd(s_used, 1) : TB_POOL;
+      if (slot < TB_POOL) {
+        const T wv = __ldg(o.src_w + d * o.w_stride + (long long)k * n_comp + comp);
+        const T* sg = o.signals + (long long)__ldg(o.src_sig + k) * o.src_steps + step0;
+        s_pool[TS * TB_POOL + slot] = __ldg(o.src_mul + k);
+#pragma unroll
+        for (int s = 0; s < TS; ++s)
+          s_pool[s * TB_POOL + slot] = mul_rn(wv, step0 + s < o.src_steps ? __ldg(sg + s) : T(0));
+      } else {
+        slot = -2 - min(k - sk0, 32000);
+        src_many = true;
       }
+      w_src[i * TBW + col] = (short)slot;
+    });
+  }
+  // Monitors sample owned cells: the warp stages the lanes x rows that hold its points each
+  // sub-step (record 10 values a pair of cells), and the block writes the points from there.
+  // A warp whose points spread over more cells than it can stage writes row by row.
+  if (mk0 < mk1) {
+    const int c0 = X0 + HX, c1 = min(X0 + TBW - HX, nx);
+    for (int k = mk0 + lane; k < mk1; k += 32) {
+      const int c = __ldg(o.mon_cell + k), y = c / nx, x = c - y * nx;
+      if (x < c0 || x >= c1) continue;
+      mon_rows |= 1u << (y - yb);
+      mon_lanes |= 1u << ((x - X0) >> 1);
+    }
+    mon_rows = __reduce_or_sync(FULL, mon_rows);
+    mon_lanes = __reduce_or_sync(FULL, mon_lanes);
+    const int n_rec = __popc(mon_rows) * __popc(mon_lanes);
+    if (lane == 0 && n_rec > 0) rec0 = atomicAdd(s_used + 2, n_rec);
+    rec0 = __shfl_sync(FULL, rec0, 0);
+    mon_staged = n_rec > 0 && rec0 + n_rec <= TB_REC;
+    mon_direct = n_rec > 0 && !mon_staged;
+    for (int k = mk0 + lane; k < mk1 && mon_staged; k += 32) {
+      const int c = __ldg(o.mon_cell + k), y = c / nx, x = c - y * nx;
+      if (x < c0 || x >= c1) continue;
+      const int slot = atomicAdd(s_used + 1, 1), ln = (x - X0) >> 1;
+      const int rec = __popc(mon_rows & ((1u << (y - yb)) - 1u)) * __popc(mon_lanes) + __popc(mon_lanes & ((1u << ln) - 1u));
+      if (slot < TB_POINTS) s_list[slot] = make_int2((rec0 + rec) * 10 + ((x - X0) & 1), __ldg(o.mon_point + k));
+      else mon_direct = true;  // the list is full: the warp's points are also written row by row
+    }
+    mon_direct = __any_sync(FULL, mon_direct);
+  }
+  src_many = __any_sync(FULL, src_many);
+  const bool own = lane >= HX / 2 && lane < 32 - HX / 2 && xa < nx;
+  // owned cells inside the capture box: bit 2*i + column
+  unsigned cap = 0u;
+  if (o.region != nullptr && own) {
+    const int rx = xa - o.rx0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int tr = tr0 + i, y = yb + i, ry = y - o.ry0;
+      if (tr < TS || tr >= TH - TS || y >= ny || ry < 0 || ry >= o.rh) continue;
+      if (rx >= 0 && rx < o.rw) cap |= 1u << (2 * i);
+      if (xa + 1 < nx && rx + 1 >= 0 && rx + 1 < o.rw) cap |= 2u << (2 * i);
     }
   }
+
+  // Factors, where any tile cell has loss or lies on or outside the grid's edge. Cells
+  // whose H or E the reference never changes (Hx in the last column, Hy in the last
+  // row, E on the PEC ring, everything outside) get factors that keep the value.
+  bool lossy = !inner;
+#pragma unroll
+  for (int i = 0; i < R; ++i) lossy = lossy || nonzero2(ls[i]);
+  lossy = __syncthreads_or(lossy);
+  if (lossy) {
+    const bool in0 = xa >= 0 && xa < nx, in1 = xa >= 0 && xa + 1 < nx;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int y = yb + i;
+      const bool iny = y >= 0 && y < ny, inh = y >= 0 && y < ny - 1, inty = y >= 1 && y <= ny - 2;
+      const bool i0 = inty && xa >= 1 && xa <= nx - 2, i1 = inty && xa + 1 >= 1 && xa + 1 <= nx - 2;
+      T fh0, fh1, cx0, cx1, cy0, cy1;
+      h_coeffs(lo2(ls[i]), g.chx, g.chy, fh0, cx0, cy0);  // divisions: rows free of loss skip them
+      h_coeffs(hi2(ls[i]), g.chx, g.chy, fh1, cx1, cy1);
+      const T fe0 = i0 ? sub_rn(T(1), mul_rn(mul_rn(lo2(ls[i]), lo2(cc[i])), g.inv_kd2)) : T(1);
+      const T fe1 = i1 ? sub_rn(T(1), mul_rn(mul_rn(hi2(ls[i]), hi2(cc[i])), g.inv_kd2)) : T(1);
+      cc[i] = mk2(i0 ? lo2(cc[i]) : T(0), i1 ? hi2(cc[i]) : T(0));
+      V* q = s_fac + (tr0 + i) * 32 + lane;
+      q[0] = mk2(fh0, fh1);
+      q[TH * 32] = mk2(iny && in0 && xa < nx - 1 ? -cx0 : T(0), iny && in1 && xa + 1 < nx - 1 ? -cx1 : T(0));
+      q[2 * TH * 32] = mk2(inh && in0 ? cy0 : T(0), inh && in1 ? cy1 : T(0));
+      q[3 * TH * 32] = mk2(fe0, fe1);
+    }
+  }
+  // one = 1 in a register the compiler cannot see through: x + y as fma(1, x, y), so that a
+  // product y is rounded before the sum, as in every other kernel of this update
+  const V one = mk2(g.one, g.one), mcx = mk2(-g.chx, -g.chx), pcy = mk2(g.chy, g.chy), qy = mk2(g.qy, g.qy);
+  const V zero = mk2(T(0), T(0));
+  const int n_list = min(s_used[1], TB_POINTS);  // after the barrier above: every warp has added its points
+  int ring_slot = o.n_mon > 0 && o.ring ? (int)(step0 % o.ring_len) : 0;  // of step0, then of each sub-step
+  // Writes point p of the cell at q (pairs of Ez, Hx, Hy, Hy of the row above; Hx left of the
+  // pair) to the record and the DFT ring.
+  auto write_point = [&](const T* q, int j, long long p, long long step, int slot) {
+    if (o.record != nullptr && step >= o.rec_step0 && step < o.rec_step0 + o.n_rec)
+      put3(o.record + (((step - o.rec_step0) * n_planes + dc) * o.n_mon + p) * 3, q[j], q[2 + j], q[4 + j]);
+    if (o.ring)
+      put5(o.ring + (((long long)slot * n_planes + dc) * o.n_mon + p) * 5, q[j], q[2 + j], j ? q[2] : q[8], q[4 + j],
+           q[6 + j]);
+  };
+  auto write_list = [&](int s) {  // the staged points of sub-step s, one a thread
+    const T* q = s_rec + (s & 1) * TB_REC * 10;
+    for (int i = threadIdx.x; i < n_list; i += 32 * NW) {
+      const int2 e = s_list[i];
+      const int j = e.x & 1;
+      write_point(q + e.x - j, j, e.y, step0 + s, ring_slot);
+    }
+  };
 
 #pragma unroll 1
   for (int s = 0; s < TS; ++s) {
-    const long long step = step0 + s;
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int k = 0; k < NC; ++k) s_top[w][k][j * 32 + lane] = ez[0][j][k];
-    __syncthreads();
-    // H update: Ez(x+1) by shuffle, Ez(y+1) from the next row (or warp)
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-#pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        const T r0 = __shfl_sync(FULL, ez[i][0][k], (lane + 1) & 31);
-        const T r1 = __shfl_sync(FULL, ez[i][1][k], (lane + 1) & 31);
-        T er[2], ed[2];
-        er[0] = lane == 31 ? r1 : r0;  // right of column 31 is column 32
-        er[1] = r1;                    // lane 31: beyond the tile (stale halo)
-        if (i + 1 < R) {
-          ed[0] = ez[i + 1][0][k];
-          ed[1] = ez[i + 1][1][k];
-        } else if (w + 1 < NW) {
-          ed[0] = s_top[w + 1][k][lane];
-          ed[1] = s_top[w + 1][k][32 + lane];
-        } else {
-          ed[0] = ed[1] = T(0);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          hx[i][j][k] = hx_update(fh[i][j], hx[i][j][k], cx[i][j], er[j], ez[i][j][k]);
-          hy[i][j][k] = hy_update(fh[i][j], hy[i][j][k], cy[i][j], ed[j], ez[i][j][k]);
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int k = 0; k < NC; ++k) s_bot[w][k][j * 32 + lane] = hy[R - 1][j][k];
-    __syncthreads();
-    // E update (interior): Hx(x-1) by shuffle, Hy(y-1) from the previous row (or warp)
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-#pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        const T l0 = __shfl_sync(FULL, hx[i][0][k], (lane + 31) & 31);
-        const T l1 = __shfl_sync(FULL, hx[i][1][k], (lane + 31) & 31);
-        T hl[2], hu[2];
-        hl[0] = l0;  // lane 0: beyond the tile (stale halo)
-        hl[1] = lane == 0 ? l0 : l1;
-        if (i > 0) {
-          hu[0] = hy[i - 1][0][k];
-          hu[1] = hy[i - 1][1][k];
-        } else if (w > 0) {
-          hu[0] = s_bot[w - 1][k][lane];
-          hu[1] = s_bot[w - 1][k][32 + lane];
-        } else {
-          hu[0] = hu[1] = T(0);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-          ez[i][j][k] = ez_update(fe[i][j], ez[i][j][k], cc[i][j], g.qy, hx[i][j][k], hl[j], hy[i][j][k], hu[j]);
-      }
-    }
-    // Sources (helper.py:5-118), in operation order per cell
-    if (src_rows) {
+    V* ex = s_ex + (s & 1) * (2 * NW * 32) + lane;
+    ex[w * 32] = ez[0];
+    ex[(NW + w) * 32] = ez[R - 1];
+    __syncthreads();  // also orders the factors before their first use, and the staged samples
+    if (n_list > 0 && s > 0) write_list(s - 1);
+    if (s > 0 && ++ring_slot == o.ring_len) ring_slot = 0;  // now the slot of sub-step s
+    const V ez_dn = w + 1 < NW ? ex[(w + 1) * 32] : zero;
+    const V ez_up = w > 0 ? ex[(NW + w - 1) * 32] : zero;
+    V hu;  // new Hy of the row above the current one
+    if (!lossy) {
+      hyu = fma2(one, hyu, mul2(pcy, sub2(ez[0], ez_up)));
+      hu = hyu;
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        if (!(src_rows & (1u << i))) continue;  // uniform across the warp
-        const int y = yb + i;
-        const int k0 = s_src[w * R + i][0], k1 = s_src[w * R + i][1];
-        for (int kk = k0; kk < k1; ++kk) {
-          const int xo = __ldg(o.src_cell + kk) - y * nx;
-          if (xo != xs[0] && xo != xs[1]) continue;
-          const T m = __ldg(o.src_mul + kk);
-          const int sg = __ldg(o.src_sig + kk);
-          const T sv = (step < o.src_steps) ? __ldg(o.signals + (long long)sg * o.src_steps + step) : T(0);
+        const V down = i + 1 < R ? ez[i + 1 < R ? i + 1 : i] : ez_dn;
+        const V er = mk2(hi2(ez[i]), __shfl_down_sync(FULL, lo2(ez[i]), 1));  // lane 31: stale halo
+        hx[i] = fma2(one, hx[i], mul2(mcx, sub2(er, ez[i])));
+        hy[i] = fma2(one, hy[i], mul2(pcy, sub2(down, ez[i])));
+        const V hl = mk2(__shfl_up_sync(FULL, hi2(hx[i]), 1), lo2(hx[i]));  // lane 0: stale halo
+        ez[i] = fma2(one, ez[i], mul2(cc[i], fma2(qy, sub2(hy[i], hu), sub2(hl, hx[i]))));
+        hu = hy[i];
+      }
+    } else {
+      const V* q = s_fac + tr0 * 32 + lane;
+      if (w > 0) hyu = fma2(q[-32], hyu, mul2(q[2 * TH * 32 - 32], sub2(ez[0], ez_up)));
+      hu = hyu;
 #pragma unroll
-          for (int k = 0; k < NC; ++k) {
-            const T wv = __ldg(o.src_w + d * o.w_stride + (long long)kk * NC + k);
+      for (int i = 0; i < R; ++i) {
+        const V fh = q[i * 32], cx = q[(TH + i) * 32], cy = q[(2 * TH + i) * 32], fe = q[(3 * TH + i) * 32];
+        const V down = i + 1 < R ? ez[i + 1 < R ? i + 1 : i] : ez_dn;
+        const V er = mk2(hi2(ez[i]), __shfl_down_sync(FULL, lo2(ez[i]), 1));
+        hx[i] = fma2(fh, hx[i], mul2(cx, sub2(er, ez[i])));
+        hy[i] = fma2(fh, hy[i], mul2(cy, sub2(down, ez[i])));
+        const V hl = mk2(__shfl_up_sync(FULL, hi2(hx[i]), 1), lo2(hx[i]));
+        ez[i] = fma2(fe, ez[i], mul2(cc[i], fma2(qy, sub2(hy[i], hu), sub2(hl, hx[i]))));
+        hu = hy[i];
+      }
+    }
+    if (!(src_rows | mon_rows | cap)) continue;
+    const long long step = step0 + s;
+    // Sources (helper.py:5-118), in operation order per cell
+    if (src_rows) {
+      const T* add = s_pool + s * TB_POOL;
+      const T* fac = s_pool + TS * TB_POOL;
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-              if (xo == xs[j]) ez[i][j][k] = fma_rn(m, ez[i][j][k], mul_rn(wv, sv));
+      for (int i = 0; i < R; ++i) {  // no branches: rows without sources have empty maps
+        const short2 e = *reinterpret_cast<const short2*>(w_src + i * TBW + 2 * lane);
+        const int e0 = max((int)e.x, 0), e1 = max((int)e.y, 0);
+        const T v0 = lo2(ez[i]), v1 = hi2(ez[i]);
+        const T n0 = fma_rn(fac[e0], v0, add[e0]), n1 = fma_rn(fac[e1], v1, add[e1]);
+        ez[i] = mk2(e.x >= 0 ? n0 : v0, e.y >= 0 ? n1 : v1);
+      }
+      if (src_many) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          if (!(src_rows & (1u << i))) continue;
+          T v[2] = {lo2(ez[i]), hi2(ez[i])};
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int e = w_src[i * TBW + 2 * lane + j], cell = (yb + i) * nx + xa + j;
+            if (e >= -1) continue;
+            int k = sk0 + (-2 - e);
+            while (__ldg(o.src_cell + k) != cell) ++k;
+            do {
+              const T sv = step < o.src_steps ? __ldg(o.signals + (long long)__ldg(o.src_sig + k) * o.src_steps + step) : T(0);
+              v[j] = fma_rn(__ldg(o.src_mul + k), v[j],
+                            mul_rn(__ldg(o.src_w + d * o.w_stride + (long long)k * n_comp + comp), sv));
+              ++k;
+            } while (k < sk1 && __ldg(o.src_cell + k) == cell);
           }
+          ez[i] = mk2(v[0], v[1]);
         }
       }
     }
@@ -479,81 +676,76 @@ __global__ void __launch_bounds__(32 * NW) step2d_tb_kernel(
     if (cap) {
       const long long slot = step + 1 - o.reg_step0;
       if (slot >= 1 && slot < o.n_reg) {
+        T* q = o.region + ((slot * n_planes + dc) * o.rh + (yb - o.ry0)) * (long long)o.rw + (xa - o.rx0);
 #pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            if (cap & (1u << (i * 2 + j))) {
-              const int rx = xs[j] - o.rx0, ry = yb + i - o.ry0;
-#pragma unroll
-              for (int k = 0; k < NC; ++k)
-                o.region[(((slot * g.n_designs + d) * NC + k) * o.rh + ry) * (long long)o.rw + rx] = ez[i][j][k];
-            }
+        for (int i = 0; i < R; ++i) {
+          if (cap & (1u << (2 * i))) q[i * o.rw] = lo2(ez[i]);
+          if (cap & (2u << (2 * i))) q[i * o.rw + 1] = hi2(ez[i]);
+        }
       }
     }
-    // Monitor samples of owned cells: record and DFT ring
+    // Monitor samples of owned cells, with Hx left of each pair
     if (mon_rows) {
-      const long long slot = o.ring != nullptr ? step % o.ring_len : 0;
-      const bool rec = o.record != nullptr && step >= o.rec_step0 && step < o.rec_step0 + o.n_rec;
+      T side[R];
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        if (!(mon_rows & (1u << i))) continue;  // uniform across the warp
-        const int y = yb + i;
-        T hl[2][NC], hu[2][NC];
+      for (int i = 0; i < R; ++i) side[i] = __shfl_up_sync(FULL, hi2(hx[i]), 1);
+      if (mon_staged && (mon_lanes >> lane & 1u)) {
+        T* q = s_rec + ((s & 1) * TB_REC + rec0 + __popc(mon_lanes & ((1u << lane) - 1u))) * 10;
 #pragma unroll
-        for (int k = 0; k < NC; ++k) {
-          const T l0 = __shfl_sync(FULL, hx[i][0][k], (lane + 31) & 31);
-          const T l1 = __shfl_sync(FULL, hx[i][1][k], (lane + 31) & 31);
-          hl[0][k] = l0;
-          hl[1][k] = lane == 0 ? l0 : l1;
-#pragma unroll
-          for (int j = 0; j < 2; ++j) hu[j][k] = i > 0 ? hy[i - 1][j][k] : (w > 0 ? s_bot[w - 1][k][j * 32 + lane] : T(0));
+        for (int i = 0; i < R; ++i) {
+          if (!(mon_rows & (1u << i))) continue;  // uniform across the warp
+          V* v = reinterpret_cast<V*>(q);
+          v[0] = ez[i];
+          v[1] = hx[i];
+          v[2] = hy[i];
+          v[3] = yb + i < 1 ? zero : (i > 0 ? hy[i > 0 ? i - 1 : 0] : hyu);
+          q[8] = xa >= 1 ? side[i] : T(0);
+          q += __popc(mon_lanes) * 10;
         }
-        const int k0 = s_mon[w * R + i][0], k1 = s_mon[w * R + i][1];
-        for (int kk = k0; kk < k1; ++kk) {
-          const int xo = __ldg(o.mon_cell + kk) - y * nx;
-          const int p = __ldg(o.mon_point + kk);
+      }
+      if (mon_direct) {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            if (xo != xs[j] || !own[j]) continue;
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-              if (rec) {
-                T* dst = o.record + ((((step - o.rec_step0) * g.n_designs + d) * NC + k) * (long long)o.n_mon + p) * 3;
-                dst[0] = ez[i][j][k];
-                dst[1] = hx[i][j][k];
-                dst[2] = hy[i][j][k];
-              }
-              if (o.ring) {
-                T* q = o.ring + (((slot * g.n_designs + d) * NC + k) * (long long)o.n_mon + p) * 5;
-                q[0] = ez[i][j][k];
-                q[1] = hx[i][j][k];
-                q[2] = xo >= 1 ? hl[j][k] : T(0);
-                q[3] = hy[i][j][k];
-                q[4] = y >= 1 ? hu[j][k] : T(0);
-              }
-            }
+        for (int i = 0; i < R; ++i) {
+          if (!(mon_rows & (1u << i))) continue;
+          const V up = yb + i < 1 ? zero : (i > 0 ? hy[i > 0 ? i - 1 : 0] : hyu);
+          const T hl = xa >= 1 ? side[i] : T(0);
+          const int base = (yb + i) * nx;
+          for (int k = mk0; k < mk1; ++k) {  // every lane reads the list, the owner writes
+            const int x = __ldg(o.mon_cell + k) - base;
+            if (x != xa && x != xa + 1) continue;
+            if (!own) continue;
+            const T q[9] = {lo2(ez[i]), hi2(ez[i]), lo2(hx[i]), hi2(hx[i]), lo2(hy[i]), hi2(hy[i]), lo2(up), hi2(up), hl};
+            if (x == xa) write_point(q, 0, __ldg(o.mon_point + k), step, ring_slot);
+            else write_point(q, 1, __ldg(o.mon_point + k), step, ring_slot);
           }
         }
       }
     }
   }
+  if (n_list > 0) {  // uniform across the block
+    __syncthreads();
+    write_list(TS - 1);
+  }
   // Store the owned box
+  if (!own) return;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const int tr = w * R + i, y = yb + i;
+    const int tr = tr0 + i, y = yb + i;
     if (tr < TS || tr >= TH - TS || y >= ny) continue;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int x = xs[j];
-      if (!own[j]) continue;
-      const long long r = (long long)y * pitch + x;
-#pragma unroll
-      for (int k = 0; k < NC; ++k) {
-        const long long off = fb + k * g.plane + r;
-        ez_out[off] = ez[i][j][k];
-        if (x < nx - 1) hx_out[off] = hx[i][j][k];
-        if (y < ny - 1) hy_out[off] = hy[i][j][k];
+    const long long off = fb + i * pitch;
+    if (vec && xa + 1 < nx - 1) {  // both columns exist in every component
+      *reinterpret_cast<V*>(ez_out + off) = ez[i];
+      *reinterpret_cast<V*>(hx_out + off) = hx[i];
+      if (y < ny - 1) *reinterpret_cast<V*>(hy_out + off) = hy[i];
+    } else {
+      const bool in1 = xa + 1 < nx;
+      ez_out[off] = lo2(ez[i]);
+      if (in1) ez_out[off + 1] = hi2(ez[i]);
+      if (xa < nx - 1) hx_out[off] = lo2(hx[i]);
+      if (xa + 1 < nx - 1) hx_out[off + 1] = hi2(hx[i]);
+      if (y < ny - 1) {
+        hy_out[off] = lo2(hy[i]);
+        if (in1) hy_out[off + 1] = hi2(hy[i]);
       }
     }
   }
@@ -572,6 +764,7 @@ Geo2D<T> make_geo(const bz_grid2d* gd) {
   g.chy = (T)gd->chy;
   g.qy = (T)gd->qy;
   g.inv_kd2 = (T)gd->inv_kd2;
+  g.one = (T)1;
   return g;
 }
 
@@ -603,10 +796,21 @@ Ops2D<T> make_ops(const bz_source_ops* s, const bz_monitor_ops* m) {
   return o;
 }
 
-template <typename T, int NC, int TS, int R, int NW>
+template <typename T, int TS, int R, int NW, int MINB>
 int launch_tb(const bz_grid2d* gd, const bz_fields2d* f, const bz_source_ops* s, const bz_monitor_ops* m,
               int64_t step, const int64_t* d_step, cudaStream_t st) {
-  constexpr int OW = 64 - 2 * TS, OH = NW * R - 2 * TS;
+  constexpr int OW = TBW - 2 * (TS + 1), OH = NW * R - 2 * TS;
+  constexpr int SMEM = TbSmem<T, TS, R, NW>::BYTES;
+  const auto kernel = step2d_tb_kernel<T, TS, R, NW, MINB>;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return fail(BZ_ERR_CUDA, "bz_step2d_multi: no current device");
+  static std::atomic<unsigned long long> opted{0ull};  // devices whose limit is raised (bit per ordinal below 64)
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (!(opted.load() & bit)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+      return fail(BZ_ERR_CUDA, "bz_step2d_multi: cannot configure the kernel's shared memory");
+    opted.fetch_or(bit);
+  }
   const Geo2D<T> g = make_geo<T>(gd);
   Ops2D<T> o = make_ops<T>(s, m);
   if (m && m->region && m->n_reg > 1) {
@@ -618,41 +822,51 @@ int launch_tb(const bz_grid2d* gd, const bz_fields2d* f, const bz_source_ops* s,
     o.n_reg = m->n_reg;
     o.reg_step0 = m->reg_step0;
   }
+  uintptr_t bits = (uintptr_t)f->ce | (uintptr_t)f->loss;
+  for (int i = 0; i < 2; ++i) bits |= (uintptr_t)f->ez[i] | (uintptr_t)f->hx[i] | (uintptr_t)f->hy[i];
+  const bool vec = bits % (2 * sizeof(T)) == 0;  // pairs start at even columns and the pitch is even
   const int src = (int)(step & 1);
-  dim3 grid((unsigned)ceil_div(gd->nx, OW), (unsigned)ceil_div(gd->ny, OH), (unsigned)gd->n_designs);
-  step2d_tb_kernel<T, NC, TS, R, NW><<<grid, 32 * NW, 0, st>>>(
-      (const T*)f->ez[src], (const T*)f->hx[src], (const T*)f->hy[src], (T*)f->ez[src ^ 1], (T*)f->hx[src ^ 1],
-      (T*)f->hy[src ^ 1], (const T*)f->ce, (const T*)f->loss, g, o, (long long)step, (const long long*)d_step);
+  const int n_planes = gd->n_designs * gd->n_comp;
+  for (int p0 = 0; p0 < n_planes; p0 += 65535) {  // the z extent of a grid is at most 65535
+    dim3 grid((unsigned)ceil_div(gd->nx, OW), (unsigned)ceil_div(gd->ny, OH),
+              (unsigned)(n_planes - p0 < 65535 ? n_planes - p0 : 65535));
+    kernel<<<grid, 32 * NW, SMEM, st>>>(
+        (const T*)f->ez[src], (const T*)f->hx[src], (const T*)f->hy[src], (T*)f->ez[src ^ 1], (T*)f->hx[src ^ 1],
+        (T*)f->hy[src ^ 1], (const T*)f->ce, (const T*)f->loss, g, o, gd->n_comp, p0, n_planes, vec,
+        (long long)step, (const long long*)d_step);
+  }
   return check_launch("bz_step2d_multi");
 }
 
-// Tile shapes: 1 = 4 rows x 8 warps, 2 = 4 rows x 16 warps, 3 = 8 rows x 8 warps,
-// 4 = 5 rows x 16 warps, 5 = 6 rows x 12 warps (float, one component); wider types
-// use 2 rows x 16 warps.
-template <typename T, int NC, int TS>
+// Tile shapes (rows a warp x warps) for float: 0, 2 and 5 = 8 x 8, 1 = 4 x 8, 3 = 2 x 16,
+// 4 = 4 x 12; three steps a launch always take 4 x 8 (a shape costs little
+// there). Double takes 4 x 16, or 2 x 16 for tiles 1 and 3.
+template <typename T, int TS>
 int tb_by_tile(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* s, const bz_monitor_ops* m,
                int64_t step, int32_t tile, const int64_t* d_step, cudaStream_t st) {
-  if constexpr (sizeof(T) == 4 && NC == 1) {
+  if constexpr (sizeof(T) == 4 && TS == 3) {
+    return launch_tb<T, TS, 4, 8, 3>(g, f, s, m, step, d_step, st);
+  } else if constexpr (sizeof(T) == 4) {
     switch (tile) {
-      case 1: return launch_tb<T, NC, TS, 4, 8>(g, f, s, m, step, d_step, st);
-      case 3: return launch_tb<T, NC, TS, 8, 8>(g, f, s, m, step, d_step, st);
-      case 4: return launch_tb<T, NC, TS, 5, 16>(g, f, s, m, step, d_step, st);
-      case 5: return launch_tb<T, NC, TS, 6, 12>(g, f, s, m, step, d_step, st);
-      default: return launch_tb<T, NC, TS, 4, 16>(g, f, s, m, step, d_step, st);
+      case 1: return launch_tb<T, TS, 4, 8, 3>(g, f, s, m, step, d_step, st);
+      case 3: return launch_tb<T, TS, 2, 16, 2>(g, f, s, m, step, d_step, st);
+      case 4: return launch_tb<T, TS, 4, 12, 2>(g, f, s, m, step, d_step, st);
+      default: return launch_tb<T, TS, 8, 8, 2>(g, f, s, m, step, d_step, st);
     }
   } else {
-    return launch_tb<T, NC, TS, 2, 16>(g, f, s, m, step, d_step, st);
+    if (tile == 1 || tile == 3) return launch_tb<T, TS, 2, 16, 1>(g, f, s, m, step, d_step, st);
+    return launch_tb<T, TS, 4, 16, 1>(g, f, s, m, step, d_step, st);
   }
 }
 
-template <typename T, int NC>
+template <typename T>
 int tb_by_steps(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* s, const bz_monitor_ops* m,
                 int64_t step, int32_t n_sub, int32_t tile, const int64_t* d_step, cudaStream_t st) {
   switch (n_sub) {
-    case 3: return tb_by_tile<T, NC, 3>(g, f, s, m, step, tile, d_step, st);
-    case 7: return tb_by_tile<T, NC, 7>(g, f, s, m, step, tile, d_step, st);
-    case 9: return tb_by_tile<T, NC, 9>(g, f, s, m, step, tile, d_step, st);
-    default: return tb_by_tile<T, NC, 5>(g, f, s, m, step, tile, d_step, st);
+    case 3: return tb_by_tile<T, 3>(g, f, s, m, step, tile, d_step, st);
+    case 7: return tb_by_tile<T, 7>(g, f, s, m, step, tile, d_step, st);
+    case 9: return tb_by_tile<T, 9>(g, f, s, m, step, tile, d_step, st);
+    default: return tb_by_tile<T, 5>(g, f, s, m, step, tile, d_step, st);
   }
 }
 
@@ -756,9 +970,6 @@ extern "C" int bz_step2d_multi(const bz_grid2d* g, const bz_fields2d* f, const b
   if (f->power != nullptr)
     return bz::fail(BZ_ERR_UNSUPPORTED, "bz_step2d_multi: power accumulation needs bz_step2d");
   cudaStream_t st = bz::as_stream(stream);
-  if (g->dtype == BZ_F32)
-    return g->n_comp == 1 ? bz::tb_by_steps<float, 1>(g, f, s, m, step, n_sub, tile, d_step, st)
-                          : bz::tb_by_steps<float, 2>(g, f, s, m, step, n_sub, tile, d_step, st);
-  return g->n_comp == 1 ? bz::tb_by_steps<double, 1>(g, f, s, m, step, n_sub, tile, d_step, st)
-                        : bz::tb_by_steps<double, 2>(g, f, s, m, step, n_sub, tile, d_step, st);
+  return g->dtype == BZ_F32 ? bz::tb_by_steps<float>(g, f, s, m, step, n_sub, tile, d_step, st)
+                            : bz::tb_by_steps<double>(g, f, s, m, step, n_sub, tile, d_step, st);
 }

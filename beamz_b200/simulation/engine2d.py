@@ -22,8 +22,10 @@ from .guard import DivergenceGuard
 
 GRAPH_CHUNK = 64  # at most this many steps per captured graph
 RING_LEN = GRAPH_CHUNK  # monitor samples kept between DFT folds
-# (steps per launch, register-tile shape) tried by the autotuner
-TUNE_CANDIDATES = ((9, 0), (9, 5), (7, 0), (7, 4), (7, 5), (7, 1), (7, 3), (5, 0), (5, 4), (5, 1), (3, 1))
+# (steps per launch, register-tile shape) tried by the autotuner: the large tile for grids
+# that fill the GPU several times over, smaller ones (less halo work per block, more
+# blocks) for grids that do not
+TUNE_CANDIDATES = ((9, 0), (7, 0), (5, 0), (9, 4), (7, 4), (9, 1), (7, 1), (5, 1), (9, 3), (7, 3))
 _TUNED: dict = {}  # (device name, nx, ny, designs, components, dtype) -> (time_block, tb_tile)
 
 

@@ -179,6 +179,53 @@ def test_time_blocked_batch_matches_single_steps(bz, precision):
         assert rel_l2(dft, outs[0][1]) <= 1e-12
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,lossy", [(61, 47, True), (170, 215, False), (171, 214, True), (300, 130, True), (2, 2, False)])
+def test_blocked_tiles_match_single_steps(bz, nx, ny, lossy, precision):
+    """Every tile shape against single steps, bit for bit: grids with tiles clear of loss
+    and of the edges, loss on two sides, line sources along both axes with cells shared by
+    two signals, points shared by crossing lines, and more points and source cells in a
+    tile than it holds on chip."""
+    from beamz_b200.devices.sources import ModeSource
+    from beamz_b200.simulation.engine2d import Engine2D
+
+    rng = np.random.default_rng(nx + ny)
+    eps = 1.0 + 11.0 * rng.random((ny, nx))
+    sigma = np.zeros((ny, nx))
+    if lossy:
+        sigma[:, :9] = 2e5 * rng.random((ny, 9))
+        sigma[-7:, :] = 1e5 * rng.random((7, nx))
+    dx = 20e-9
+    dt = 0.99 * dx / (299792458.0 * np.sqrt(2))
+    n = 63
+    t = np.arange(n) * dt
+    sig = np.sin(2 * np.pi * 1.9e14 * t + 0.3)
+
+    def line(points, direction, signal):
+        src = ModeSource.__new__(ModeSource)
+        src.__dict__.update(direction=direction, enforce_direction=True, signal=signal, mode_profiles=[
+            [[rng.standard_normal(), x * dx, y * dx, 0.0] for x, y in points]])
+        return src
+
+    xs, ys = nx // 2, ny // 2
+    srcs = [line([(xs, y) for y in range(ny)], "+x", sig), line([(x, ys) for x in range(nx)], "-y", sig[::-1] + 0.5j * sig),
+            bz.GaussianSource(position=(xs * dx, ys * dx), width=5 * dx, signal=sig)]
+    freqs = [1.9e14]
+    mons = [bz.Monitor(start=(0, y * dx), end=((nx - 1) * dx, y * dx), frequencies=freqs)
+            for y in (0, ny - 1, *range(ys, min(ys + 9, ny)))]
+    mons += [bz.Monitor(start=(x * dx, 0), end=(x * dx, (ny - 1) * dx), frequencies=freqs) for x in (0, nx - 1, xs)]
+    outs = []
+    for tb, tile in ((1, 0), (3, 0), (5, 0), (7, 0), (9, 0), (7, 1), (9, 3), (5, 4), (9, 4)):
+        eng = Engine2D(eps, sigma, dx, dx, dt, n, srcs, mons, precision=precision, n_comp=2, record=True,
+                       use_graphs=False, time_block=tb, tb_tile=tile)
+        eng.run_steps(n)
+        outs.append(([eng.field(k).cpu().numpy() for k in ("Ez", "Hx", "Hy")] + [eng.take_records()], eng.dft_fields()))
+    for exact, dft in outs[1:]:
+        for a, b in zip(exact, outs[0][0]):
+            np.testing.assert_array_equal(a, b)
+        assert rel_l2(dft, outs[0][1]) <= 1e-12
+
+
 def test_graph_replay_equals_direct_launches(bz):
     eps, sigma, dx, dt, t, sig, _ = _random_problem(5, n_steps=300)
     src = bz.GaussianSource(position=(18 * dx, 14 * dx), width=dx / 10, signal=sig)
