@@ -17,14 +17,15 @@
 // the kernel accumulates grad += -e*(E_{n+1} - E_n)/eps_r from captured forward
 // fields. The post phase then prepares the input of step n-1:
 //   e_{n-1} = mul*(dJ/dE_n + objective term), through the same source operations.
-#include "bz_stencil.cuh"
+#include <atomic>
+
+#include "bz_tile.cuh"
 
 namespace bz {
 namespace {
 
 constexpr int BX = 128;
 constexpr int RB = 16;
-constexpr unsigned FULL = 0xffffffffu;
 
 template <typename T>
 struct AdjArgs {
@@ -184,200 +185,311 @@ __global__ void __launch_bounds__(BX) adjoint2d_kernel(AdjArgs<T> a, long long s
 
 
 // ---- several reverse steps per launch (temporal blocking) ---------------------------
-// The register tile of the forward step2d_tb kernel, run backwards: a block holds 64
-// columns x NW*R rows (lane l: columns X0+l and X0+32+l) with the per-cell factors, and
-// performs TS reverse steps m = step, step-1, ..., each one the single-step adjoint
-// above: gradient from the incoming e on owned cells of the design box (applied after
-// the last sub-step from a shared-memory history of those e), U = Ce*e, the
-// H-like pass (U(x+1) by shuffle, U(y+1) from the next row or warp), the E-like pass
-// (wx(x-1) by shuffle, wy(y-1) from the previous row or warp), carried fh*hx', fh*hy',
-// then the operations preparing step m-1 on every tile cell. Boundary rules enter the
-// factors (Ce = 0, Fe = 1 off the interior; cx = 0 in the last column and outside,
-// cy = 0 in the last row and outside), and the stale halo of TS cells is not stored.
+// The register tile of the blocked forward kernel (bz_step2d.cu: two adjacent columns a
+// lane as one packed operand, R rows a warp, halo of TS+1 columns and TS rows a side),
+// run backwards: TS reverse steps m = step, step-1, ..., each the single-step adjoint
+// above. Per sub-step a warp receives U = Ce*e of the rows above and below it (one block
+// barrier) and carries hy' of the row above itself. Tiles clear of loss and off the
+// grid's edge need no factor but Ce; there the E-like pass takes the constant factors out
+// of the differences (cx*(hx'(x) - hx'(x-1))). Other tiles read fh, cx, cy and Fe from
+// shared memory; boundary rules enter the factors (Ce = 0, Fe = 1 off the interior;
+// cx = 0 in the last column and outside, cy = 0 in the last row and outside).
+//
+// Design-box cells keep each sub-step's incoming e in shared memory ([TS][R][thread]
+// pairs); their gradient terms are applied after the last sub-step, off the
+// barrier-paced loop. The history and the factors share one region, so that two float
+// blocks of five steps fit an SM; a tile that needs both (the box next to the absorber)
+// recomputes its factors from the loss each sub-step instead.
+//
+// Bound by issue and latency like the forward kernel, and by the tile loads, which two
+// blocks an SM hide only in part. 64 designs of 600 x 400 with a 120 x 120 box, 1500
+// reverse steps: 98 ms in launches of five (two blocks an SM), 124 ms in launches of seven
+// (one block: the history takes 115 KB); 114 ms before, with seven factors and fields a
+// cell in registers and two barriers a sub-step.
+constexpr int ADJ_POOL = 160;  // cells with operations held on chip; further ones are read from memory
 template <typename T, int TS, int R, int NW>
-__global__ void __launch_bounds__(32 * NW) adjoint2d_tb_kernel(AdjArgs<T> a, long long step0) {
-  constexpr int TW = 64, TH = NW * R, OW = TW - 2 * TS, OH = TH - 2 * TS;
-  static_assert(TS % 2 == 1 && OH > 0 && R * 2 <= 32, "bad temporal tile");
+struct AdjSmem {
+  static constexpr int TH = NW * R;
+  static constexpr int FAC = 4 * TH * TBW * (int)sizeof(T), HIST = TS * TH * TBW * (int)sizeof(T);
+  static constexpr int SHARED = FAC > HIST ? FAC : HIST;
+  static constexpr int EXCH = 2 * 2 * NW * TBW * (int)sizeof(T);
+  static constexpr int POOL = (TS + 1) * ADJ_POOL * (int)sizeof(T);
+  static constexpr int MAP = TH * TBW * (int)sizeof(short);
+  static constexpr int BYTES = SHARED + EXCH + POOL + MAP + 16;
+};
+
+// The operations of one cell (sorted list entries k .. until another cell) at the N steps
+// sstep, sstep-1, ...: v <- fac * v + add[i].
+template <int N, typename T>
+__device__ __forceinline__ void adj_run(const AdjArgs<T>& a, int d, int k, int k1, long long sstep, T& fac, T (&add)[N]) {
+  const int cell = __ldg(a.src_cell + k);
+  fac = T(1);
+#pragma unroll
+  for (int i = 0; i < N; ++i) add[i] = T(0);
+  do {
+    const T m = __ldg(a.src_mul + k), wv = __ldg(a.src_w + d * a.w_stride + k);
+    const T* sg = a.signals + (long long)__ldg(a.src_sig + k) * a.src_steps + sstep;
+    fac *= m;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      add[i] = m * add[i] + wv * (sstep - i >= 0 && sstep - i < a.src_steps ? __ldg(sg - i) : T(0));
+    ++k;
+  } while (k < k1 && __ldg(a.src_cell + k) == cell);
+}
+
+template <typename T, int TS, int R, int NW, int MINB>
+__global__ void __launch_bounds__(32 * NW, MINB) adjoint2d_tb_kernel(AdjArgs<T> a, bool vec, long long step0) {
+  typedef typename PairOf<T>::type V;
+  typedef AdjSmem<T, TS, R, NW> S;
+  constexpr int TH = S::TH, HX = TS + 1, OW = TBW - 2 * HX, OH = TH - 2 * TS, NT = 32 * NW;
+  static_assert(TS % 2 == 1 && OW > 0 && OH > 0 && R <= 16, "bad temporal tile");
+  extern __shared__ __align__(16) unsigned char adj_smem[];
+  V* s_fac = reinterpret_cast<V*>(adj_smem);   // [4][TH][32]: fh, cx, cy, Fe
+  V* s_hist = s_fac;                           // or [TS][R][NT]: incoming e of design-box cells
+  V* s_ex = reinterpret_cast<V*>(adj_smem + S::SHARED);                 // [2][2][NW][32]: first, last rows' U
+  T* s_pool = reinterpret_cast<T*>(adj_smem + S::SHARED + S::EXCH);     // [TS + 1][ADJ_POOL]: addends, factor
+  int* s_used = reinterpret_cast<int*>(s_pool + (TS + 1) * ADJ_POOL);
+  short* s_map = reinterpret_cast<short*>(s_used + 4);                  // [TH][64]
+
   const int nx = a.nx, ny = a.ny, pitch = a.pitch;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.z;
-  const int X0 = (int)blockIdx.x * OW - TS, Y0 = (int)blockIdx.y * OH - TS;
-  const int yb = Y0 + w * R;
-  const long long fb = (long long)d * a.plane;
-  const long long mb = (a.n_mat > 1 ? (long long)d : 0LL) * a.plane;
-  __shared__ T s_top[NW][TW], s_bot[NW][TW];
-  __shared__ int s_src[TH][2];
+  const int X0 = (int)blockIdx.x * OW - HX, Y0 = (int)blockIdx.y * OH - TS;
+  const int yb = Y0 + w * R, xa = X0 + 2 * lane, tr0 = w * R;
+  const long long fb = (long long)d * a.plane + (long long)yb * pitch + xa;  // the thread's first cell
+  const long long mb = (a.n_mat > 1 ? (long long)d : 0LL) * a.plane + (long long)yb * pitch + xa;
+  const bool inner = X0 >= 1 && X0 + TBW - 1 <= nx - 2 && Y0 >= 1 && Y0 + TH - 1 <= ny - 2;
+  const bool in0 = xa >= 0 && xa < nx, in1 = xa >= 0 && xa + 1 < nx;
 
-  int xs[2];
-  xs[0] = X0 + lane;
-  xs[1] = X0 + 32 + lane;
-  T e[R][2], hx[R][2], hy[R][2], fh[R][2], cx[R][2], cy[R][2], Fe[R][2], Ce[R][2];
+  int sk0 = 0, sk1 = 0;  // the operations of the warp's rows
+  if (a.n_src > 0 && max(yb, 0) < min(yb + R, ny)) {
+    sk0 = __ldg(a.src_row + max(yb, 0));
+    sk1 = __ldg(a.src_row + min(yb + R, ny));
+  }
+  if (threadIdx.x == 0) *s_used = 0;
+
+  V e[R], hx[R], hy[R], cc[R], ls[R];
+  V hyu;  // hy of the row above the warp's first; stale, as all halo rows, for warp 0
+  if (inner && vec) {
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int y = yb + i;
+    for (int i = 0; i < R; ++i) {
+      const int r = i * pitch;
+      ls[i] = ldg2(a.loss + mb + r);
+      e[i] = ldg2(a.e_in + fb + r);
+      hx[i] = ldg2(a.hx_in + fb + r);
+      hy[i] = ldg2(a.hy_in + fb + r);
+      cc[i] = ldg2(a.ce + mb + r);
+    }
+    hyu = ldg2(a.hy_in + fb - pitch);
+  } else {
+    const bool inm0 = in0 && xa < nx - 1, inm1 = in1 && xa + 1 < nx - 1;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int x = xs[j];
-      const bool in = x >= 0 && x < nx && y >= 0 && y < ny;
-      const long long r = in ? (long long)y * pitch + x : 0LL;
-      const T ls = in ? __ldg(a.loss + mb + r) : T(0), c = in ? __ldg(a.ce + mb + r) : T(0);
-      h_coeffs(ls, a.chx, a.chy, fh[i][j], cx[i][j], cy[i][j]);
-      const bool interior = x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2;
-      Fe[i][j] = interior ? T(1) - ls * c * a.inv_kd2 : T(1);
-      Ce[i][j] = interior ? c : T(0);
-      if (!(in && x < nx - 1)) cx[i][j] = T(0);
-      if (!(in && y < ny - 1)) cy[i][j] = T(0);
-      e[i][j] = in ? __ldg(a.e_in + fb + r) : T(0);
-      hx[i][j] = (in && x < nx - 1) ? __ldg(a.hx_in + fb + r) : T(0);
-      hy[i][j] = (in && y < ny - 1) ? __ldg(a.hy_in + fb + r) : T(0);
+    for (int i = 0; i < R; ++i) {
+      const int y = yb + i, r = i * pitch;
+      const bool iny = y >= 0 && y < ny, inh = y >= 0 && y < ny - 1;
+      ls[i] = ld_pair(a.loss + mb + r, in0 && iny, in1 && iny);
+      e[i] = ld_pair(a.e_in + fb + r, in0 && iny, in1 && iny);
+      hx[i] = ld_pair(a.hx_in + fb + r, inm0 && iny, inm1 && iny);
+      hy[i] = ld_pair(a.hy_in + fb + r, in0 && inh, in1 && inh);
+      cc[i] = ld_pair(a.ce + mb + r, in0 && iny, in1 && iny);
+    }
+    hyu = ld_pair(a.hy_in + fb - pitch, in0 && yb >= 1 && yb < ny, in1 && yb >= 1 && yb < ny);
+  }
+  __syncthreads();  // the pool's counter is set
+
+  // Operations on every tile cell: a map cell -> pool slot, -1 for none, -2 - n for a cell
+  // beyond the pool, found from the warp's n-th list entry on.
+  unsigned src_rows = 0u;
+  bool src_many = false;
+  short* const w_src = s_map + tr0 * TBW;
+  if (sk0 < sk1) {
+    for (int i = lane; i < R * TBW; i += 32) w_src[i] = -1;
+    __syncwarp();
+    src_rows = scan_ops(a.src_cell, sk0, sk1, nx, yb, X0, max(X0, 0), min(X0 + TBW, nx), lane,
+                        [&](int i, int col, int k, bool) {
+      int slot = atomicAdd(s_used, 1);
+      if (slot < ADJ_POOL) {
+        T fac, add[TS];
+        adj_run<TS>(a, d, k, sk1, step0 - 1, fac, add);
+#pragma unroll
+        for (int s = 0; s < TS; ++s) s_pool[s * ADJ_POOL + slot] = add[s];
+        s_pool[TS * ADJ_POOL + slot] = fac;
+      } else {
+        slot = -2 - min(k - sk0, 32000);
+        src_many = true;
+      }
+      w_src[i * TBW + col] = (short)slot;
+    });
+  }
+  src_many = __any_sync(FULL, src_many);
+  const bool own = lane >= HX / 2 && lane < 32 - HX / 2 && xa < nx;
+  unsigned gbits = 0u;  // owned design-box cells: bit 2*i + column
+  if (a.grad != nullptr && own) {
+    const int rx = xa - a.rx0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int tr = tr0 + i, y = yb + i, ry = y - a.ry0;
+      if (tr < TS || tr >= TH - TS || y >= ny || ry < 0 || ry >= a.rh) continue;
+      if (rx >= 0 && rx < a.rw) gbits |= 1u << (2 * i);
+      if (xa + 1 < nx && rx + 1 >= 0 && rx + 1 < a.rw) gbits |= 2u << (2 * i);
     }
   }
-  if (lane < R) {  // operation ranges of the tile's rows over its columns
-    const int y = yb + lane, tr = w * R + lane;
-    int s0 = 0, s1 = 0;
-    if (a.n_src > 0 && y >= 0 && y < ny) {
-      const int lo = __ldg(a.src_row + y), hi = __ldg(a.src_row + y + 1);
-      if (lo < hi) {
-        s0 = lower_bound_i(a.src_cell, lo, hi, y * nx + max(X0, 0));
-        s1 = lower_bound_i(a.src_cell, s0, hi, y * nx + min(X0 + TW, nx));
+
+  bool lossy = !inner;
+#pragma unroll
+  for (int i = 0; i < R; ++i) lossy = lossy || nonzero2(ls[i]);
+  lossy = __syncthreads_or(lossy);
+  const bool boxed = __syncthreads_or(gbits != 0u);
+  // factors of row yb + i (i = -1: the row above, fh and cy only); Ce of the row given
+  auto factors = [&](int i, V c, V l, V& fh, V& cx, V& cy, V& fe) {
+    const int y = yb + i;
+    const bool iny = y >= 0 && y < ny, inh = y >= 0 && y < ny - 1;
+    T fh0, fh1, cx0, cx1, cy0, cy1;
+    h_coeffs(lo2(l), a.chx, a.chy, fh0, cx0, cy0);
+    h_coeffs(hi2(l), a.chx, a.chy, fh1, cx1, cy1);
+    fh = mk2(fh0, fh1);
+    cx = mk2(iny && in0 && xa < nx - 1 ? cx0 : T(0), iny && in1 && xa + 1 < nx - 1 ? cx1 : T(0));
+    cy = mk2(inh && in0 ? cy0 : T(0), inh && in1 ? cy1 : T(0));
+    fe = mk2(T(1) - lo2(l) * lo2(c) * a.inv_kd2, T(1) - hi2(l) * hi2(c) * a.inv_kd2);  // 1 where c = 0
+  };
+  if (lossy) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int y = yb + i;
+      const bool inty = y >= 1 && y <= ny - 2;
+      cc[i] = mk2(inty && xa >= 1 && xa <= nx - 2 ? lo2(cc[i]) : T(0),
+                  inty && xa + 1 >= 1 && xa + 1 <= nx - 2 ? hi2(cc[i]) : T(0));
+      if (!boxed) {
+        V fh, cx, cy, fe;
+        factors(i, cc[i], ls[i], fh, cx, cy, fe);
+        V* q = s_fac + (tr0 + i) * 32 + lane;
+        q[0] = fh;
+        q[TH * 32] = cx;
+        q[2 * TH * 32] = cy;
+        q[3 * TH * 32] = fe;
       }
     }
-    s_src[tr][0] = s0;
-    s_src[tr][1] = s1;
   }
-  __syncwarp();
-  unsigned src_rows = 0u, gbits = 0u;
-  bool own[2];
-  own[0] = lane >= TS && xs[0] < nx;
-  own[1] = lane < 32 - TS && xs[1] < nx;
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    if (s_src[w * R + i][0] < s_src[w * R + i][1]) src_rows |= 1u << i;
-    const int tr = w * R + i, y = yb + i;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int rx = xs[j] - a.rx0, ry = y - a.ry0;
-      if (a.grad != nullptr && own[j] && tr >= TS && tr < TH - TS && y < ny && rx >= 0 && rx < a.rw && ry >= 0 &&
-          ry < a.rh)
-        gbits |= 1u << (i * 2 + j);
-    }
-  }
-
-  // Design-box cells keep each sub-step's incoming e here ([TS][R][2][thread]); the
-  // gradient terms are applied after the last sub-step, off the barrier-paced loop.
-  extern __shared__ __align__(16) unsigned char s_hist_raw[];
-  T* s_hist = reinterpret_cast<T*>(s_hist_raw);
-  constexpr int NT = 32 * NW;
+  const V one = mk2(T(1), T(1)), qy = mk2(a.qy, a.qy), mqy = mk2(-a.qy, -a.qy), zero = mk2(T(0), T(0));
+  const V pcx = mk2(a.chx, a.chx), pcy = mk2(a.chy, a.chy);
 
 #pragma unroll 1
   for (int s = 0; s < TS; ++s) {
-    const long long m = step0 - s;  // reverse step taken by this sub-step
     if (gbits) {
 #pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-          if (gbits & (1u << (i * 2 + j))) s_hist[((s * R + i) * 2 + j) * NT + threadIdx.x] = e[i][j];
+      for (int i = 0; i < R; ++i) s_hist[(s * R + i) * NT + threadIdx.x] = e[i];
     }
-    T U[R][2];
+    V* ex = s_ex + (s & 1) * (2 * NW * 32) + lane;
+    V U = mul2(cc[0], e[0]);
+    ex[w * 32] = U;
+    ex[(NW + w) * 32] = mul2(cc[R - 1], e[R - 1]);
+    __syncthreads();  // also orders the factors before their first use
+    const V u_dn = w + 1 < NW ? ex[(w + 1) * 32] : zero;
+    const V u_up = w > 0 ? ex[(NW + w - 1) * 32] : zero;
+    if (!lossy) {
+      hyu = fma2(mqy, sub2(U, u_up), hyu);
+      V hu = hyu;  // hy' of the row above
 #pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) U[i][j] = Ce[i][j] * e[i][j];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) s_top[w][j * 32 + lane] = U[0][j];
-    __syncthreads();
-    // H-like pass: hx' = hx + U(x+1) - U(x), hy' = hy - qy*(U(y+1) - U(y))
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const T r0 = __shfl_sync(FULL, U[i][0], (lane + 1) & 31);
-      const T r1 = __shfl_sync(FULL, U[i][1], (lane + 1) & 31);
-      T ur[2], ud[2];
-      ur[0] = lane == 31 ? r1 : r0;
-      ur[1] = r1;
-      if (i + 1 < R) {
-        ud[0] = U[i + 1][0];
-        ud[1] = U[i + 1][1];
-      } else if (w + 1 < NW) {
-        ud[0] = s_top[w + 1][lane];
-        ud[1] = s_top[w + 1][32 + lane];
-      } else {
-        ud[0] = ud[1] = T(0);
+      for (int i = 0; i < R; ++i) {
+        const V un = i + 1 < R ? mul2(cc[i + 1 < R ? i + 1 : i], e[i + 1 < R ? i + 1 : i]) : u_dn;
+        const V ur = mk2(hi2(U), __shfl_down_sync(FULL, lo2(U), 1));  // lane 31: stale halo
+        hx[i] = fma2(one, hx[i], sub2(ur, U));
+        hy[i] = fma2(mqy, sub2(un, U), hy[i]);
+        const V hl = mk2(__shfl_up_sync(FULL, hi2(hx[i]), 1), lo2(hx[i]));  // lane 0: stale halo
+        e[i] = fma2(pcx, sub2(hx[i], hl), fma2(pcy, sub2(hu, hy[i]), e[i]));
+        hu = hy[i];
+        U = un;
+      }
+    } else {
+      const V* q = s_fac + tr0 * 32 + lane;
+      V wu = zero;  // cy * hy' of the row above
+      if (w > 0) {
+        V fh, cx, cy, fe;
+        if (boxed) {
+          factors(-1, zero, ld_pair(a.loss + mb - pitch, in0 && yb >= 1 && yb <= ny, in1 && yb >= 1 && yb <= ny), fh, cx, cy, fe);
+        } else {
+          fh = q[-32];
+          cy = q[2 * TH * 32 - 32];
+        }
+        hyu = fma2(mqy, sub2(U, u_up), hyu);
+        wu = mul2(cy, hyu);
+        hyu = mul2(fh, hyu);
       }
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        hx[i][j] = hx[i][j] + (ur[j] - U[i][j]);         // hx'
-        hy[i][j] = hy[i][j] - a.qy * (ud[j] - U[i][j]);  // hy'
+      for (int i = 0; i < R; ++i) {
+        V fh, cx, cy, fe;
+        if (boxed) {
+          const bool iny = yb + i >= 0 && yb + i < ny;
+          factors(i, cc[i], ld_pair(a.loss + mb + i * pitch, in0 && iny, in1 && iny), fh, cx, cy, fe);
+        } else {
+          fh = q[i * 32];
+          cx = q[(TH + i) * 32];
+          cy = q[(2 * TH + i) * 32];
+          fe = q[(3 * TH + i) * 32];
+        }
+        const V un = i + 1 < R ? mul2(cc[i + 1 < R ? i + 1 : i], e[i + 1 < R ? i + 1 : i]) : u_dn;
+        const V ur = mk2(hi2(U), __shfl_down_sync(FULL, lo2(U), 1));
+        const V hxp = fma2(one, hx[i], sub2(ur, U)), hyp = fma2(mqy, sub2(un, U), hy[i]);
+        const V wx = mul2(cx, hxp), wy = mul2(cy, hyp);
+        const V wl = mk2(__shfl_up_sync(FULL, hi2(wx), 1), lo2(wx));
+        e[i] = fma2(one, fma2(fe, e[i], sub2(wx, wl)), sub2(wu, wy));
+        hx[i] = mul2(fh, hxp);
+        hy[i] = mul2(fh, hyp);
+        wu = wy;
+        U = un;
       }
     }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) s_bot[w][j * 32 + lane] = cy[R - 1][j] * hy[R - 1][j];
-    __syncthreads();
-    // E-like pass: e_prev = Fe*e - (wx(x-1) - wx) + (wy(y-1) - wy); carried fh*h'
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      T wx[2], wy[2], wl[2], wu[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        wx[j] = cx[i][j] * hx[i][j];
-        wy[j] = cy[i][j] * hy[i][j];
-      }
-      const T l0 = __shfl_sync(FULL, wx[0], (lane + 31) & 31);
-      const T l1 = __shfl_sync(FULL, wx[1], (lane + 31) & 31);
-      wl[0] = l0;
-      wl[1] = lane == 0 ? l0 : l1;
-      if (i > 0) {
-        wu[0] = cy[i - 1][0] * hy[i - 1][0];
-        wu[1] = cy[i - 1][1] * hy[i - 1][1];
-      } else if (w > 0) {
-        wu[0] = s_bot[w - 1][lane];
-        wu[1] = s_bot[w - 1][32 + lane];
-      } else {
-        wu[0] = wu[1] = T(0);
-      }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) e[i][j] = Fe[i][j] * e[i][j] - (wl[j] - wx[j]) + (wu[j] - wy[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        hx[i][j] = fh[i][j] * hx[i][j];
-        hy[i][j] = fh[i][j] * hy[i][j];
-      }
     // operations preparing step m-1 (none after step 0)
-    if (src_rows && m >= 1) {
-      const long long sstep = m - 1;
+    if (src_rows && step0 - s >= 1) {
+      const T* add = s_pool + s * ADJ_POOL;
+      const T* fac = s_pool + TS * ADJ_POOL;
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         if (!(src_rows & (1u << i))) continue;  // uniform across the warp
-        const int y = yb + i;
-        const int k0 = s_src[w * R + i][0], k1 = s_src[w * R + i][1];
-        for (int kk = k0; kk < k1; ++kk) {
-          const int xo = __ldg(a.src_cell + kk) - y * nx;
-          if (xo != xs[0] && xo != xs[1]) continue;
-          const T sv =
-              sstep < a.src_steps ? __ldg(a.signals + (long long)__ldg(a.src_sig + kk) * a.src_steps + sstep) : T(0);
-          const T mul = __ldg(a.src_mul + kk), wv = __ldg(a.src_w + d * a.w_stride + kk);
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            if (xo == xs[j]) e[i][j] = mul * e[i][j] + wv * sv;
+        const short2 m = *reinterpret_cast<const short2*>(w_src + i * TBW + 2 * lane);
+        const int m0 = max((int)m.x, 0), m1 = max((int)m.y, 0);
+        T v0 = lo2(e[i]), v1 = hi2(e[i]);
+        if (m.x >= 0) v0 = fac[m0] * v0 + add[m0];
+        if (m.y >= 0) v1 = fac[m1] * v1 + add[m1];
+        if (src_many) {
+          const int cell = (yb + i) * nx + xa;
+          T f, ad[1];
+          if (m.x < -1) {
+            int k = sk0 - 2 - m.x;
+            while (__ldg(a.src_cell + k) != cell) ++k;
+            adj_run<1>(a, d, k, sk1, step0 - s - 1, f, ad);
+            v0 = f * v0 + ad[0];
+          }
+          if (m.y < -1) {
+            int k = sk0 - 2 - m.y;
+            while (__ldg(a.src_cell + k) != cell + 1) ++k;
+            adj_run<1>(a, d, k, sk1, step0 - s - 1, f, ad);
+            v1 = f * v1 + ad[0];
+          }
         }
+        e[i] = mk2(v0, v1);
       }
     }
   }
+  if (!own) return;
   // store the owned box
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const int tr = w * R + i, y = yb + i;
+    const int tr = tr0 + i, y = yb + i;
     if (tr < TS || tr >= TH - TS || y >= ny) continue;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int x = xs[j];
-      if (!own[j]) continue;
-      const long long r = fb + (long long)y * pitch + x;
-      a.e_out[r] = e[i][j];
-      if (x < nx - 1) a.hx_out[r] = hx[i][j];
-      if (y < ny - 1) a.hy_out[r] = hy[i][j];
+    const long long off = fb + i * pitch;
+    if (vec && xa + 1 < nx - 1) {  // both columns exist in every component
+      *reinterpret_cast<V*>(a.e_out + off) = e[i];
+      *reinterpret_cast<V*>(a.hx_out + off) = hx[i];
+      if (y < ny - 1) *reinterpret_cast<V*>(a.hy_out + off) = hy[i];
+    } else {
+      a.e_out[off] = lo2(e[i]);
+      if (in1) a.e_out[off + 1] = hi2(e[i]);
+      if (xa < nx - 1) a.hx_out[off] = lo2(hx[i]);
+      if (xa + 1 < nx - 1) a.hx_out[off + 1] = hi2(hx[i]);
+      if (y < ny - 1) {
+        a.hy_out[off] = lo2(hy[i]);
+        if (in1) a.hy_out[off + 1] = hi2(hy[i]);
+      }
     }
   }
   // grad -= sum over the sub-steps' reverse steps m of e_m * (E_{m+1} - E_m), over
@@ -385,26 +497,32 @@ __global__ void __launch_bounds__(32 * NW) adjoint2d_tb_kernel(AdjArgs<T> a, lon
   if (gbits) {
     const long long per = (long long)a.n_designs * a.rh * a.rw, db = (long long)d * a.rh * a.rw;
     const long long eb = (a.n_mat > 1 ? (long long)d : 0LL) * a.rh * a.rw;
+    const long long p0 = step0 + 1 - a.fwd_step0;  // captured plane E_{m+1} of sub-step 0
+    const bool all = p0 < a.n_fwd && p0 - TS >= 0;  // every plane the sub-steps need was captured
 #pragma unroll
-    for (int i = 0; i < R; ++i)
+    for (int i = 0; i < R; ++i) {
+      if (!(gbits >> (2 * i) & 3u)) continue;
+      const long long cell = (long long)(yb + i - a.ry0) * a.rw + (xa - a.rx0);
+      const bool g0 = gbits >> (2 * i) & 1u, g1 = gbits >> (2 * i) & 2u;
+      const T* f = a.fwd + p0 * per + db + cell;
+      T f0[TS + 1], f1[TS + 1];  // planes p0, p0-1, ..., p0-TS, all loads issued before the sums
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        if (!(gbits & (1u << (i * 2 + j)))) continue;
-        const long long cell = (long long)(yb + i - a.ry0) * a.rw + (xs[j] - a.rx0);
-        const long long p0 = step0 + 1 - a.fwd_step0;  // captured plane E_{m+1} of sub-step 0
-        T f[TS + 1];  // planes p0, p0-1, ..., p0-TS, all loads issued before the sums
-#pragma unroll
-        for (int k = 0; k <= TS; ++k)
-          f[k] = (p0 - k >= 0 && p0 - k < a.n_fwd) ? a.fwd[(p0 - k) * per + db + cell] : T(0);
-        const double er = a.eps_region[eb + cell];
-        const double gv = a.grad[db + cell];
-        T acc = T(0);  // the block's terms in the fields' precision (e and the planes are T)
-#pragma unroll
-        for (int s = 0; s < TS; ++s)
-          if (p0 - s >= 1 && p0 - s < a.n_fwd)
-            acc += s_hist[((s * R + i) * 2 + j) * NT + threadIdx.x] * (f[s] - f[s + 1]);
-        a.grad[db + cell] = gv - (double)acc / er;
+      for (int k = 0; k <= TS; ++k) {
+        const bool ok = all || (p0 - k >= 0 && p0 - k < a.n_fwd);
+        f0[k] = ok && g0 ? __ldg(f - k * per) : T(0);
+        f1[k] = ok && g1 ? __ldg(f - k * per + 1) : T(0);
       }
+      T acc0 = T(0), acc1 = T(0);  // the block's terms in the fields' precision (e and the planes are T)
+#pragma unroll
+      for (int s = 0; s < TS; ++s)
+        if (p0 - s >= 1 && p0 - s < a.n_fwd) {
+          const V h = s_hist[(s * R + i) * NT + threadIdx.x];
+          acc0 += lo2(h) * (f0[s] - f0[s + 1]);
+          acc1 += hi2(h) * (f1[s] - f1[s + 1]);
+        }
+      if (g0) a.grad[db + cell] -= (double)acc0 / a.eps_region[eb + cell];
+      if (g1) a.grad[db + cell + 1] -= (double)acc1 / a.eps_region[eb + cell + 1];
+    }
   }
 }
 
@@ -465,18 +583,26 @@ int launch_adj(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops* o
 template <typename T, int TS>
 int launch_adj_tb(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops* ops, int64_t step, int32_t phase,
                   cudaStream_t st) {
-  constexpr int R = sizeof(T) == 4 ? 4 : 2, NW = 16;
-  constexpr int hist = TS * R * 2 * 32 * NW * (int)sizeof(T);  // at most 147 KB (TS = 9)
+  // float: 64 x 64 tiles, two blocks an SM up to five steps; double: 64 x 32
+  constexpr int R = sizeof(T) == 4 ? 8 : 2, NW = sizeof(T) == 4 ? 8 : 16;
+  constexpr int SMEM = AdjSmem<T, TS, R, NW>::BYTES, MINB = sizeof(T) == 4 ? 2 : 1;
+  const auto kernel = adjoint2d_tb_kernel<T, TS, R, NW, MINB>;
   const AdjArgs<T> a = adj_args<T>(g, s, ops, phase);
-  dim3 grid((unsigned)ceil_div(g->nx, 64 - 2 * TS), (unsigned)ceil_div(g->ny, NW * R - 2 * TS), (unsigned)g->n_designs);
-  static bool opted = false;  // history plus the static tiles pass the default 48 KB
-  if (!opted) {
-    if (cudaFuncSetAttribute(adjoint2d_tb_kernel<T, TS, R, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, hist) !=
-        cudaSuccess)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return fail(BZ_ERR_CUDA, "bz_adjoint_step2d_multi: no current device");
+  static std::atomic<unsigned long long> opted{0ull};  // devices whose limit is raised (bit per ordinal below 64)
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (!(opted.load() & bit)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
       return fail(BZ_ERR_CUDA, "bz_adjoint_step2d_multi: cannot configure the kernel's shared memory");
-    opted = true;
+    opted.fetch_or(bit);
   }
-  adjoint2d_tb_kernel<T, TS, R, NW><<<grid, 32 * NW, a.grad ? hist : 0, st>>>(a, (long long)step);
+  uintptr_t bits = (uintptr_t)s->ce | (uintptr_t)s->loss;
+  for (int i = 0; i < 2; ++i) bits |= (uintptr_t)s->e[i] | (uintptr_t)s->hx[i] | (uintptr_t)s->hy[i];
+  const bool vec = bits % (2 * sizeof(T)) == 0;
+  dim3 grid((unsigned)ceil_div(g->nx, TBW - 2 * (TS + 1)), (unsigned)ceil_div(g->ny, NW * R - 2 * TS),
+            (unsigned)g->n_designs);
+  kernel<<<grid, 32 * NW, SMEM, st>>>(a, vec, (long long)step);
   return check_launch("bz_adjoint_step2d_multi");
 }
 

@@ -294,30 +294,30 @@ class AdjointFDTD2D:
         torch.cuda.current_stream().synchronize()
         return grad.cpu().numpy() / self._adj_scale[:, None, None]
 
-    def _time_adjoint(self, grid, state, stream, reps: int = 3) -> int:
-        """Blocked or single reverse steps, whichever runs faster on this problem (a
-        single design on a small grid leaves the blocked tiles too few to fill the GPU).
-        Timed before the backward pass: no gradient, no operations, and every launch reads
-        the still-zero current copy, so nothing changes."""
+    def _time_adjoint(self, grid, state, stream, reps: int = 2) -> int:
+        """Reverse steps per launch, the fastest on this problem: blocked launches (the
+        forward run's block, or a shorter one, whose gradient history is small enough for
+        two blocks per SM) or single steps (a single design on a small grid leaves the
+        blocked tiles too few to fill the GPU). Timed before the backward pass, with the
+        gradient history allocated and no operations; every launch reads the still-zero
+        current copy and only adds zeros to the gradient, so nothing changes."""
         tb = self.engine.time_block
         if tb <= 1:
             return 1
-        grad = state.grad
-        state.grad = None
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         best = {}
-        for k in (tb, 1):
-            nat.adjoint_step2d_multi(grid, state, None, tb - 1, k, 0, stream)  # warm-up
+        for k in sorted({tb, min(tb, 5), 1}, reverse=True):
+            n = 4 if k == 1 else 1
             t = float("inf")
-            for _ in range(reps):
+            for r in range(reps + 1):  # the first one warms up
                 a.record()
-                for _ in range(tb // k):
-                    nat.adjoint_step2d_multi(grid, state, None, tb - 1, k, 0, stream)
+                for _ in range(n):
+                    nat.adjoint_step2d_multi(grid, state, None, k - 1, k, 0, stream)
                 b.record()
                 b.synchronize()
-                t = min(t, a.elapsed_time(b))
+                if r > 0:
+                    t = min(t, a.elapsed_time(b) / (n * k))
             best[k] = t
-        state.grad = grad
         return min(best, key=best.get)
 
     def value_and_grad(self, eps_region):
