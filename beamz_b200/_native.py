@@ -116,6 +116,8 @@ _step2d = _sig("bz_step2d", C.c_int, [C.POINTER(Grid2D), C.POINTER(Fields2D), C.
                                        C.POINTER(MonitorOps), i64, vp, vp])
 _step2d_multi = _sig("bz_step2d_multi", C.c_int, [C.POINTER(Grid2D), C.POINTER(Fields2D), C.POINTER(SourceOps),
                                                    C.POINTER(MonitorOps), i64, i32, i32, vp, vp])
+_step2d_multi_power = _sig("bz_step2d_multi_power", C.c_int, [C.POINTER(Grid2D), C.POINTER(Fields2D),
+                           C.POINTER(SourceOps), C.POINTER(MonitorOps), C.c_int64, C.c_void_p, C.c_void_p])
 _dft_fold = _sig("bz_dft_fold", C.c_int, [vp, i32, i32, i64, i32, vp, i64, i64, i32, vp, vp])
 _step2d_dft_static = _sig("bz_step2d_dft_static", C.c_int,
                           [C.POINTER(Grid2D), C.POINTER(Fields2D), C.POINTER(SourceOps), C.POINTER(MonitorOps), i64,
@@ -152,7 +154,7 @@ _gemm_selftest = _sig("bz_gemm_wait_selftest", C.c_int, [vp, vp, vp, i32, vp])
 _field_check = _sig("bz_field_check", C.c_int, [vp, i32, i64, f64, i64, vp, vp])
 
 #: every symbol include/beamz_b200.h declares (checked by the CPU test suite)
-EXPORTED = ["bz_version", "bz_last_error", "bz_step2d", "bz_step2d_multi", "bz_dft_fold", "bz_step2d_dft_static", "bz_advance_step",
+EXPORTED = ["bz_version", "bz_last_error", "bz_step2d", "bz_step2d_multi", "bz_step2d_multi_power", "bz_dft_fold", "bz_step2d_dft_static", "bz_advance_step",
             "bz_adjoint_step2d", "bz_adjoint_step2d_multi", "bz_step3d", "bz_cell_ops", "bz_gather", "bz_power3d", "bz_dft_fold_q", "bz_rasterize3d", "bz_prepare_coeffs", "bz_update_h2d",
             "bz_update_e2d", "bz_rasterize2d", "bz_gemm_bf16", "bz_spectral_mix", "bz_spectral_mix_bwd", "bz_gelu_bwd",
             "bz_row_mean", "bz_row_broadcast", "bz_chan_sum", "bz_adam", "bz_to_bf16", "bz_gemm_error",
@@ -184,6 +186,11 @@ def version() -> str:
 def step2d(grid, fields, src, mon, step: int, d_step: int | None, stream: int) -> None:
     check(_step2d(C.byref(grid), C.byref(fields), C.byref(src) if src is not None else None,
                   C.byref(mon) if mon is not None else None, step, d_step, stream))
+
+
+def step2d_multi_power(grid, fields, src, mon, step: int, d_step: int | None, stream: int) -> None:
+    check(_step2d_multi_power(C.byref(grid), C.byref(fields), C.byref(src) if src is not None else None,
+                              C.byref(mon) if mon is not None else None, step, d_step, stream))
 
 
 def step2d_multi(grid, fields, src, mon, step: int, n_sub: int, tile: int, d_step: int | None, stream: int) -> None:

@@ -4,7 +4,7 @@ Holds the ping-pong field buffers ([design][component][ny][pitch], x contiguous,
 pitch a multiple of 32 elements), the update coefficients, the compiled source
 and monitor operations, and drives the step kernels: ``bz_step2d_multi`` advances
 ``time_block`` steps per launch (temporal blocking), ``bz_step2d`` one step (single
-steps, power accumulation, region capture); launches are replayed in CUDA-graph
+steps, power of complex fields); launches are replayed in CUDA-graph
 chunks when no host work is due between steps.
 """
 from __future__ import annotations
@@ -21,6 +21,7 @@ from .graphs import capture, dft_phasors
 from .guard import DivergenceGuard
 
 GRAPH_CHUNK = 64  # at most this many steps per captured graph
+POWER_BLOCK = 7  # steps of a blocked launch that accumulates power
 RING_LEN = GRAPH_CHUNK  # monitor samples kept between DFT folds
 # (steps per launch, register-tile shape) tried by the autotuner: the large tile for grids
 # that fill the GPU several times over, smaller ones (less halo work per block, more
@@ -81,8 +82,11 @@ class Engine2D:
             time_block = 7
         if int(time_block) not in (1, 3, 5, 7, 9):
             raise ValueError(f"time_block must be 1, 3, 5, 7, 9 or 'auto' (got {time_block})")
-        # power accumulation runs on the single-step kernel
-        self.time_block = 1 if power else int(time_block)
+        # power accumulation of a real field has a blocked kernel of POWER_BLOCK steps;
+        # two components are summed before squaring, which only the single-step kernel does
+        self.time_block = int(time_block)
+        if power and self.time_block > 1:
+            self.time_block = POWER_BLOCK if n_comp == 1 else 1
         self._autotune = self._autotune and not power
         self.tb_tile = int(tb_tile)
         # steps per graph: an even number of steps keeps the copy parity, so one
@@ -223,9 +227,12 @@ class Engine2D:
         timer = self.kernel_timer
         if timer is not None:
             timer.before(self.time_block)
-        nat.step2d_multi(self.grid, self._fields(), self.sops if self.sops.n_ops else None,
-                         self.mops if self.mops.n_points else None, step_arg, self.time_block, self.tb_tile,
-                         d_step_ptr, self._stream())
+        sops, mops = self.sops if self.sops.n_ops else None, self.mops if self.mops.n_points else None
+        if self.power is not None:
+            nat.step2d_multi_power(self.grid, self._fields(), sops, mops, step_arg, d_step_ptr, self._stream())
+        else:
+            nat.step2d_multi(self.grid, self._fields(), sops, mops, step_arg, self.time_block, self.tb_tile,
+                             d_step_ptr, self._stream())
         if timer is not None:
             timer.after()
 
@@ -401,6 +408,18 @@ class Engine2D:
         out = np.concatenate(self._rec_host).astype(np.float64)
         self._rec_host = []
         return out
+
+    def take_records_device(self) -> torch.Tensor | None:
+        """The samples recorded so far as a device tensor, when all of them are still there
+        (None otherwise: use take_records). Valid until the next step."""
+        if self.record is None or self._rec_host:
+            return None
+        used = self.step_index - self.mops.rec_step0
+        if used <= 0:
+            return None
+        self.mops.rec_step0 = self.step_index
+        self._graphs.clear()  # graphs bake rec_step0
+        return self.record[:used]
 
     # ---- field access ---------------------------------------------------------
     def field(self, name: str, design: int = 0) -> torch.Tensor:

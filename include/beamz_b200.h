@@ -153,13 +153,19 @@ int bz_step2d(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* src
  * monitor records and ring samples per sub-step). Each block keeps a tile of the
  * grid in registers for all sub-steps and stores the part of it that stays exact.
  * n_sub: 1, 3, 5, 7 or 9 (odd, so the copy read stays (step & 1) and the result lands
- * in copy ((step + n_sub) & 1)); 1 is bz_step2d. tile: 0 = default (4x16), 1..5 =
- * tile shapes of 4x8, 4x16, 8x8, 5x16 and 6x12 (rows per warp x warps) for float32
- * single-component fields. Region capture (mon->region) is taken per sub-step; power
- * accumulation returns BZ_ERR_UNSUPPORTED (use bz_step2d for those steps). */
+ * in copy ((step + n_sub) & 1)); 1 is bz_step2d. tile: 0 = default (8x8), 1..5 =
+ * tile shapes of 4x8, 8x8, 2x16, 4x12 and 8x8 (rows per warp x warps) for float32
+ * fields; float64 takes 4x16, or 2x16 for tiles 1 and 3. Region capture (mon->region) is
+ * taken per sub-step; power accumulation returns BZ_ERR_UNSUPPORTED (use bz_step2d or
+ * bz_step2d_multi_power for those steps). */
 int bz_step2d_multi(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* src,
                     const bz_monitor_ops* mon, int64_t step, int32_t n_sub, int32_t tile,
                     const int64_t* d_step, void* stream);
+
+/* Seven steps of bz_step2d in one launch with |S|^2 accumulation (f->power) after every
+ * one of them, as bz_step2d_multi otherwise. One component only. */
+int bz_step2d_multi_power(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* src,
+                          const bz_monitor_ops* mon, int64_t step, const int64_t* d_step, void* stream);
 
 /* Folds `count` consecutive ring samples, steps step0 .. step0+count-1 (ring slot
  * step % ring_len, count <= ring_len), into float64 DFT sums:

@@ -226,6 +226,33 @@ def test_blocked_tiles_match_single_steps(bz, nx, ny, lossy, precision):
         assert rel_l2(dft, outs[0][1]) <= 1e-12
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny", [(61, 47), (150, 131), (2, 2)])
+def test_blocked_power_matches_single_steps(bz, nx, ny, precision):
+    """|S|^2 sums, fields and records of blocked power launches against single steps
+    (whose power is added after the sources, so the sums differ by float64 rounding)."""
+    from beamz_b200.simulation.engine2d import Engine2D
+
+    rng = np.random.default_rng(nx)
+    dx = 20e-9
+    dt = 0.99 * dx / (299792458.0 * np.sqrt(2))
+    n = 24  # three blocks and three single steps
+    sigma = np.zeros((ny, nx))
+    sigma[:, :6] = 2e5
+    src = bz.GaussianSource(position=(nx // 2 * dx, ny // 2 * dx), width=dx, signal=np.sin(0.3 * np.arange(n)))
+    mon = bz.Monitor(start=(0, ny // 2 * dx), end=((nx - 1) * dx, ny // 2 * dx))
+    outs = []
+    for tb in (1, 7):
+        eng = Engine2D(1.0 + 11.0 * np.random.default_rng(1).random((ny, nx)), sigma, dx, dx, dt, n, [src], [mon],
+                       precision=precision, n_comp=1, power=True, time_block=tb)
+        eng.run_steps(n)
+        assert eng.time_block == tb
+        outs.append((eng.power_map(), eng.take_records(), eng.field("Ez").cpu().numpy()))
+    np.testing.assert_array_equal(outs[1][1], outs[0][1])
+    np.testing.assert_array_equal(outs[1][2], outs[0][2])
+    assert rel_l2(outs[1][0], outs[0][0]) <= 1e-13
+
+
 def test_graph_replay_equals_direct_launches(bz):
     eps, sigma, dx, dt, t, sig, _ = _random_problem(5, n_steps=300)
     src = bz.GaussianSource(position=(18 * dx, 14 * dx), width=dx / 10, signal=sig)
