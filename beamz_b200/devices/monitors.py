@@ -289,21 +289,24 @@ class Monitor:
             self.power_timestamps = self.power_timestamps[-n:]
 
     # ---- batch fill from the device record ----------------------------------
-    def load_record_2d(self, ez, hx, hy, times):
+    def load_record_2d(self, ez, hx, hy, times, power=None):
         """Fill fields/power from device samples [n_rec][n_points] (complex or real),
-        in one vectorised pass with the reference's per-step semantics."""
+        in one vectorised pass with the reference's per-step semantics. ``power``: the sums
+        of |S| over the steps (per point) and over the points (per step), if known."""
         if self.should_record_fields:
             self.fields["Ez"].extend(list(ez))
             self.fields["Hx"].extend(list(hx))
             self.fields["Hy"].extend(list(hy))
             self.fields["t"].extend(float(t) for t in times)
         if self.accumulate_power and len(times):
-            sx = -ez * hy
-            sy = ez * hx
-            mag = np.sqrt(sx ** 2 + sy ** 2)
-            acc = mag.sum(axis=0) if self.power_accumulated is None else self.power_accumulated + mag.sum(axis=0)
+            if power is None:
+                sx = -ez * hy
+                sy = ez * hx
+                mag = np.sqrt(sx ** 2 + sy ** 2)
+                power = mag.sum(axis=0), mag.sum(axis=1)
+            acc = power[0] if self.power_accumulated is None else self.power_accumulated + power[0]
             self.power_accumulated = acc
-            self.power_history.extend(list(mag.sum(axis=1)))
+            self.power_history.extend(list(power[1]))
             self.power_timestamps.extend(float(t) for t in times)
             self.power_accumulation_count += len(times)
         self._manage_memory()

@@ -17,15 +17,18 @@ import datetime
 from typing import Dict, Optional, Sequence
 
 import numpy as np
+import torch
 
 from ..const import EPS_0, MU_0, µm
 from ..devices.monitors import Monitor
 from ..devices.sources import GaussianSource, ModeSource
 from ..helpers import check_fdtd_stability, display_status
 from .backends import get_backend
-from .meshing import BaseMeshGrid, RegularGrid, RegularGrid3D
+from .meshing import BaseMeshGrid, RegularGrid, RegularGrid3D, to_host
 
 __all__ = ["FDTD"]
+
+PINNED_RECORD_BYTES = 128 << 20  # a monitor's samples above this go to pageable memory
 
 
 class FDTD:
@@ -245,7 +248,8 @@ class FDTD:
 
     def _collect_monitors(self):
         eng = self.engine
-        recs = eng.take_records() if hasattr(eng, "take_records") else None
+        on_device = eng.take_records_device() if hasattr(eng, "take_records_device") else None
+        recs = eng.take_records() if on_device is None and hasattr(eng, "take_records") else None
         steps = np.arange(eng.step_index)
         times = np.zeros(len(steps))
         if len(steps) > 1:
@@ -253,9 +257,37 @@ class FDTD:
         if hasattr(eng, "collect_monitors"):
             eng.collect_monitors(recs, times)
             return
-        if recs is not None:
+        if on_device is not None:
+            self._load_device_records(eng, on_device, times, steps)
+        elif recs is not None:
             self._load_records(eng, recs, times, steps)
         self._collect_dft()
+
+    def _load_device_records(self, eng, recs, times, steps):
+        """As _load_records from the device record: the samples are sorted by quantity and
+        widened to float64 on the device and arrive in page-locked memory at copy speed (a
+        four-line record of 2000 steps: 45 ms of host conversions before)."""
+        for mon, sl in zip(eng.mp.monitors, eng.mp.slices):
+            k = mon.record_interval
+            sel = slice(k - 1, None, k) if k > 1 else slice(None)
+            part = recs[sel, 0, :, sl, :].double()  # [steps][comp][points][3]
+            vals = torch.complex(part[:, 0], part[:, 1]) if eng.n_comp == 2 else part[:, 0]
+            ez, hx, hy = vals.unbind(-1)
+            mag = None
+            if mon.accumulate_power and eng.n_comp == 1 and len(times[sel]):
+                sx, sy = ez * hy, ez * hx
+                mag = torch.sqrt(sx * sx + sy * sy)
+                mag = (mag.sum(dim=0).cpu().numpy(), mag.sum(dim=1).cpu().numpy())
+            if mon.should_record_fields or (mon.accumulate_power and mag is None):
+                vals = vals.movedim(-1, 0).contiguous()
+                # page-locked memory stays locked while the caller keeps the samples
+                host = to_host(vals) if vals.nbytes <= PINNED_RECORD_BYTES else vals.cpu().numpy()
+            else:
+                host = np.zeros((3, len(times[sel]), 0))
+            eng.d2h_bytes += host.nbytes
+            mon.load_record_2d(host[0], host[1], host[2], times[sel], power=mag)
+            if len(steps[sel]):
+                mon.last_record_step = int(steps[sel][-1])
 
     def _load_records(self, eng, recs, times, steps):
         for mon, sl, ok in zip(eng.mp.monitors, eng.mp.slices, eng.mp.valid):
