@@ -221,6 +221,29 @@ __global__ void __launch_bounds__(TX * TY) step3d_kernel(Ptr3<T> in, Out3<T> out
   }
 }
 
+// Planes per block. A block walks its planes one after the other (about 2.5 planes' time
+// more for its first loads and the recomputed H plane), so a grid with few columns leaves
+// most SMs idle at 16 planes: below four waves of two blocks an SM the default takes the
+// block length with the shortest waves x (planes + 2.5), down to `least`. us a step at
+// float32, 16 / 8 planes / this rule: 100 x 50 x 29 cells 28.3 / 16.6 / 7.4 (2 planes);
+// 150 x 120 x 60 31.2 / 22.2 / 22.2 (8); 300 x 150 x 75 54.1 / 50.9 / 50.9 (8). Larger
+// grids are bound by memory and keep 16. Every length gives the same bits.
+inline int z_block(const bz_grid3d* gd, long long columns, int least) {
+  if (gd->tile_z != 0) return gd->tile_z;
+  constexpr long long WAVE = 2 * 148;
+  if (columns * ceil_div(gd->nz, 16) >= 4 * WAVE) return 16;
+  int best = 16;
+  double cost = 0.0;
+  for (int zb = 16; zb >= least; zb /= 2) {
+    const double c = (double)ceil_div(columns * ceil_div(gd->nz, zb), WAVE) * (zb + 2.5);
+    if (zb == 16 || c < cost) {
+      cost = c;
+      best = zb;
+    }
+  }
+  return best;
+}
+
 template <typename T, int NC, int ZB, int TY>
 int launch3d(const bz_grid3d* gd, const bz_fields3d* f, int64_t step, cudaStream_t st) {
   Geo3D<T> g;
@@ -672,10 +695,14 @@ int launch3d_quad(const bz_grid3d* gd, const bz_fields3d* f, int64_t step, cudaS
   }
   const int n_xt = (int)ceil_div(gd->nx, 4 * TX - 4), n_yt = (int)ceil_div(gd->ny, TY - 1);
   dim3 block(TX, TY);
-  const int zb = gd->tile_z == 8 ? 8 : 16;
+  const int zb = z_block(gd, (long long)n_xt * n_yt * gd->n_designs * gd->n_comp, 2);
   g.nzb = (int)ceil_div(gd->nz, zb);
   dim3 grid((unsigned)n_xt, (unsigned)n_yt, (unsigned)(g.nzb * gd->n_designs * gd->n_comp));
-  if (zb == 8)
+  if (zb == 2)
+    step3d_quad_kernel<2, TY><<<grid, block, 0, st>>>(in, out, (const float*)f->ce, (const float*)f->loss, g);
+  else if (zb == 4)
+    step3d_quad_kernel<4, TY><<<grid, block, 0, st>>>(in, out, (const float*)f->ce, (const float*)f->loss, g);
+  else if (zb == 8)
     step3d_quad_kernel<8, TY><<<grid, block, 0, st>>>(in, out, (const float*)f->ce, (const float*)f->loss, g);
   else
     step3d_quad_kernel<16, TY><<<grid, block, 0, st>>>(in, out, (const float*)f->ce, (const float*)f->loss, g);
@@ -699,9 +726,14 @@ inline bool pair_aligned(const bz_fields3d* f) {
 
 template <typename T, int TY>
 int dispatch3d_ty(const bz_grid3d* g, const bz_fields3d* f, int64_t step, cudaStream_t st) {
-  const bool z8 = g->tile_z == 8;  // 0 takes 16-plane z blocks
-  if (g->n_comp == 1) return z8 ? launch3d<T, 1, 8, TY>(g, f, step, st) : launch3d<T, 1, 16, TY>(g, f, step, st);
-  return z8 ? launch3d<T, 2, 8, TY>(g, f, step, st) : launch3d<T, 2, 16, TY>(g, f, step, st);
+  const long long columns = (long long)ceil_div(g->nx, TX - 1) * ceil_div(g->ny, TY - 1) * g->n_designs;
+  const int zb = z_block(g, columns, 4);
+  if (g->n_comp == 1) {
+    if (zb == 4) return launch3d<T, 1, 4, TY>(g, f, step, st);
+    return zb == 8 ? launch3d<T, 1, 8, TY>(g, f, step, st) : launch3d<T, 1, 16, TY>(g, f, step, st);
+  }
+  if (zb == 4) return launch3d<T, 2, 4, TY>(g, f, step, st);
+  return zb == 8 ? launch3d<T, 2, 8, TY>(g, f, step, st) : launch3d<T, 2, 16, TY>(g, f, step, st);
 }
 
 template <typename T>

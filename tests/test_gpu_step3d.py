@@ -257,3 +257,24 @@ def test_cross_section_mode_source_run_vs_oracle(bz):
         got = sim.engine.field(k).cpu().numpy()
         assert np.abs(got).max() > 0, k
         assert rel_l2(got, np.real(ref["fields"][k])) <= 1e-11, k
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("nx,ny,nz,n_comp", [(33, 20, 9, 1), (2, 2, 2, 1), (130, 61, 40, 1), (70, 33, 17, 2), (257, 120, 50, 1)])
+def test_default_z_blocks_match_sixteen_planes(bz, nx, ny, nz, n_comp, precision):
+    """The z block length chosen by default against 16 planes a block, bit for bit."""
+    from beamz_b200.simulation.engine3d import Engine3D
+
+    rng = np.random.default_rng(nx)
+    dx = 20e-9
+    dt = 0.99 * dx / (299792458.0 * np.sqrt(3))
+    eps = 1.0 + 11.0 * rng.random((nz, ny, nx))
+    sigma = 1e5 * rng.random((nz, ny, nx)) * (np.arange(nx) < 4)
+    src = bz.GaussianSource(position=(nx // 2 * dx, ny // 2 * dx, nz // 2 * dx), width=dx, signal=np.sin(0.3 * np.arange(12)))
+    outs = []
+    for tz in (16, 0):
+        eng = Engine3D(eps, sigma, dx, dx, dx, dt, 12, [src], [], precision=precision, n_comp=n_comp, tile_z=tz)
+        eng.run_steps(12)
+        outs.append([eng.field(k).cpu().numpy() for k in ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")])
+    for a, b in zip(*outs):
+        np.testing.assert_array_equal(a, b)
