@@ -223,15 +223,16 @@ class Engine2D:
         if timer is not None:
             timer.after()
 
-    def _launch_tb(self, step_arg: int, d_step_ptr):
+    def _launch_tb(self, step_arg: int, d_step_ptr, n_sub: int | None = None):
         timer = self.kernel_timer
+        n_sub = self.time_block if n_sub is None else n_sub
         if timer is not None:
-            timer.before(self.time_block)
+            timer.before(n_sub)
         sops, mops = self.sops if self.sops.n_ops else None, self.mops if self.mops.n_points else None
         if self.power is not None:
             nat.step2d_multi_power(self.grid, self._fields(), sops, mops, step_arg, d_step_ptr, self._stream())
         else:
-            nat.step2d_multi(self.grid, self._fields(), sops, mops, step_arg, self.time_block, self.tb_tile,
+            nat.step2d_multi(self.grid, self._fields(), sops, mops, step_arg, n_sub, self.tb_tile,
                              d_step_ptr, self._stream())
         if timer is not None:
             timer.after()
@@ -340,6 +341,8 @@ class Engine2D:
     def run_steps(self, n: int):
         """Advance n steps (see _run_steps); the E field is scanned for divergence every
         guard.every steps."""
+        if self._autotune:  # before the first interval: it sets the chunk the checks follow
+            self.autotune()
         while n > 0:
             k = min(n, max(1, self.guard.next - self.step_index))
             self._run_steps(k)
@@ -353,9 +356,9 @@ class Engine2D:
         self.guard.raise_if_diverged()
 
     def _run_steps(self, n: int):
-        """Advance n steps, replaying graph chunks where the record buffer allows."""
-        if self._autotune:
-            self.autotune()
+        """Advance n steps, replaying graph chunks where the record buffer allows. Steps left
+        over go in the longest blocked launches that fit (a single step of a small grid
+        takes longer than a block of three)."""
         while n > 0:
             self._maybe_drain()
             room = n
@@ -376,13 +379,14 @@ class Engine2D:
                 n -= self.chunk
                 self._fold()
                 continue
-            if tb > 1 and room >= tb:
-                if self.step_index - self._folded > RING_LEN - tb:
+            k = next((b for b in ((tb,) if self.power is not None else (tb, 7, 5, 3)) if 1 < b <= min(tb, room)), 1)
+            if k > 1:
+                if self.step_index - self._folded > RING_LEN - k:
                     self._fold()
-                self._launch_tb(self.step_index, None)
+                self._launch_tb(self.step_index, None, k)
                 self.n_step_launches += 1
-                self.step_index += tb
-                n -= tb
+                self.step_index += k
+                n -= k
                 continue
             self.step_once()
             n -= 1
