@@ -19,6 +19,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "bz_internal.cuh"
@@ -725,6 +726,316 @@ int launch_gemm_tma(const GemmP& p, cudaStream_t st) {
   return rc == BZ_OK ? 1 : rc;
 }
 
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+// ---- tcgen05 + TMA path on CTA pairs: 256 x 256 tiles, persistent -----------------------
+// The single-CTA kernel above reads 48 KB of operands per 128 x 256 x 64 slice, about
+// 96 bytes a clock and SM at the tensor pipe's rate: more than the L2 delivers, and its
+// epilogue leaves the pipe idle between tiles. Here two CTAs of a cluster share one
+// 256 x 256 tile (cta_group::2 MMAs of M = 256 issued by the even CTA): each loads its
+// 128 rows of A and its half of B's 256 rows, 32 KB a slice. The pairs are persistent;
+// each CTA's accumulator rows are double-buffered in TMEM (2 x 256 columns), so the four
+// epilogue warps write a tile while the next one is multiplied. Roles: warp 0 loads (six
+// 32 KB stages; both CTAs' copies complete on the even CTA's barrier), warp 1 of the even
+// CTA issues the MMAs, warps 2-5 run the epilogue. tcgen05.commit frees a stage in both
+// CTAs at once. Every output element sums its K slices in the same
+// order as in the single-CTA kernel: the same bits. Waits are bounded as above.
+// M x N x K, us, single-CTA kernel -> this one: 2048 x 1024 x 14400 in two K splits 93 ->
+// 52; 2048 x 14400 x 1024 92 -> 56; 8192 x 1024 x 14400 275 -> 179 (1350 TFLOP/s); 8192 x
+// 14400 x 1024 307 -> 194. Passing the odd CTA's landed stages on with a remote arrive
+// from one of its threads instead: 154, 115, 568, 417.
+namespace pair {
+constexpr int S = 6, BM = 256, BN = 256, BK = 64, THREADS = 192;
+constexpr int A_ST = 128 * BK * 2, STAGE = 2 * A_ST;
+constexpr int NBAR = 2 * S + 5;  // full, empty per stage; tfull[2], tempty[2], done
+constexpr int SMEM = S * STAGE + 1024 + 8 * NBAR + 16;
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}  // namespace pair
+
+// Bounded wait whose success orders what a thread of the other CTA did before its arrive.
+__device__ __forceinline__ bool tc_wait_cluster(uint32_t mbar, uint32_t parity) {
+  for (int i = 0; i < tc::WAIT_LIMIT; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// A copy into this CTA's shared memory that signals a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_mbar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
+          dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(cluster_mbar)
+      : "memory");
+}
+
+__device__ __forceinline__ void arrive_rank0(uint32_t mbar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(mbar)
+      : "memory");
+}
+
+__device__ __forceinline__ void commit_pair(uint32_t mbar) {  // the barrier at this offset in both CTAs
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(mbar),
+      "h"((uint16_t)3)
+      : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
+    gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmP p,
+                     int m_tiles, int n_tiles) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  unsigned char* bar = smem + pair::S * pair::STAGE;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 8 * pair::NBAR);
+  const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t full0 = static_cast<uint32_t>(__cvta_generic_to_shared(bar));
+  const uint32_t empty0 = full0 + 8 * pair::S, tfull0 = empty0 + 8 * pair::S;
+  const uint32_t tempty0 = tfull0 + 16, done = tempty0 + 16;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(tmem_slot))),
+                 "r"(2 * pair::BN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+  }
+  if (threadIdx.x == 32) {
+    for (int i = 0; i < pair::NBAR; ++i) {
+      const uint32_t b = full0 + 8 * i;
+      const uint32_t count = b >= tempty0 && b < done ? 8u : 1u;  // four epilogue warps of either CTA
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(b), "r"(count));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+  __syncthreads();
+  cluster_sync();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+  const uint32_t taddr = *tmem_slot;
+
+  const int ktiles = (p.K + pair::BK - 1) / pair::BK, kper = (ktiles + p.splitk - 1) / p.splitk;
+  const int total = m_tiles * n_tiles * p.splitk, first = (int)blockIdx.x >> 1, stride = (int)gridDim.x >> 1;
+  auto k_range = [&](int t, int& k0, int& k1) {  // tile t = (split, m, n), n fastest
+    const int ks = t / (m_tiles * n_tiles);
+    k0 = ks * kper;
+    k1 = min(ktiles, k0 + kper);
+  };
+  bool ok = true;
+  if (warp == 0 && lane == 0) {  // ---- loads: both CTAs' copies complete on the even CTA's barrier
+    uint32_t full_r0;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(full_r0) : "r"(full0));
+    int it = 0;
+    for (int t = first; t < total && ok; t += stride) {
+      const int mn = t % (m_tiles * n_tiles), m0 = (mn / n_tiles) * pair::BM + (int)rank * 128;
+      const int n0 = (mn % n_tiles) * pair::BN + (int)rank * 128;
+      int k0, k1;
+      k_range(t, k0, k1);
+      for (int k = k0; k < k1; ++k, ++it) {
+        const int s = it % pair::S;
+        if (it >= pair::S && !tc_wait(empty0 + 8 * s, (uint32_t)((it / pair::S - 1) & 1))) {
+          ok = false;
+          break;
+        }
+        const uint32_t st = sbase + s * pair::STAGE, fb = full_r0 + 8 * s;
+        if (rank == 0)
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full0 + 8 * s), "r"(2 * pair::STAGE)
+                       : "memory");
+        tma_load_2d_pair(st, &tmA, k * pair::BK, m0, fb);
+        tma_load_2d_pair(st + pair::A_ST, &tmB, k * pair::BK, n0, fb);
+      }
+    }
+    if (rank == 0)
+      for (int j = max(0, it - pair::S); j < it; ++j)  // all copies of both CTAs have landed before they end
+        if (!tc_wait(full0 + 8 * (j % pair::S), (uint32_t)((j / pair::S) & 1))) ok = false;
+  } else if (warp == 1 && lane == 0 && rank == 0) {
+    int it = 0, n_acc = 0;
+    for (int t = first; t < total && ok; t += stride, ++n_acc) {
+      int k0, k1;
+      k_range(t, k0, k1);
+      const int acc = n_acc & 1;
+      if (n_acc >= 2 && !tc_wait_cluster(tempty0 + 8 * acc, (uint32_t)((n_acc / 2 - 1) & 1))) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+      for (int k = k0; k < k1; ++k, ++it) {
+        const int s = it % pair::S;
+        if (!tc_wait(full0 + 8 * s, (uint32_t)((it / pair::S) & 1))) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+        const uint32_t a0 = sbase + s * pair::STAGE, b0 = a0 + pair::A_ST;
+#pragma unroll
+        for (int kk = 0; kk < pair::BK / 16; ++kk) {
+          const uint64_t da = tc_sdesc_sw128(a0 + kk * 32), db = tc_sdesc_sw128(b0 + kk * 32);
+          asm volatile(
+              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+              :
+              : "r"(taddr + (uint32_t)(acc * pair::BN)), "l"(da), "l"(db), "r"(pair::IDESC), "r"(k > k0 || kk > 0 ? 1u : 0u));
+        }
+        commit_pair(empty0 + 8 * s);
+      }
+      if (ok) commit_pair(tfull0 + 8 * acc);
+    }
+    if (!ok) {  // let issued MMAs drain before the TMEM goes
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done));
+      tc_wait(done, 0u);
+    }
+  } else if (warp >= 2) {  // ---- epilogue: warp w owns accumulator rows 32 (w % 4) ...
+    const int quad = warp & 3;
+    int n_acc = 0;
+    for (int t = first; t < total; t += stride, ++n_acc) {
+      const int acc = n_acc & 1;
+      if (!tc_wait(tfull0 + 8 * acc, (uint32_t)((n_acc / 2) & 1))) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+      const int mn = t % (m_tiles * n_tiles), n0 = (mn % n_tiles) * pair::BN;
+      const int m = (mn / n_tiles) * pair::BM + (int)rank * 128 + quad * 32 + lane;
+      for (int c0 = 0; c0 < pair::BN && n0 + c0 < p.N; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32(taddr + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * pair::BN + c0), v);
+        if (m >= p.M) continue;
+        const long long o = (long long)m * p.ldc + n0 + c0;
+        const int n = min(32, p.N - n0 - c0);
+        if (p.outh) {
+          bf16* q = p.outh + o;
+          if (n == 32) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              uint4 w4;
+              __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&w4);
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                h[i] = __floats2bfloat162_rn(p.alpha * __uint_as_float(v[8 * e + 2 * i]),
+                                             p.alpha * __uint_as_float(v[8 * e + 2 * i + 1]));
+              reinterpret_cast<uint4*>(q)[e] = w4;
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (e < n) q[e] = __float2bfloat16_rn(p.alpha * __uint_as_float(v[e]));
+          }
+        } else if (p.atomic) {
+          float* q = p.outf + o;
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            if (e + 4 <= n)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(q + e),
+                           "f"(p.alpha * __uint_as_float(v[e])), "f"(p.alpha * __uint_as_float(v[e + 1])),
+                           "f"(p.alpha * __uint_as_float(v[e + 2])), "f"(p.alpha * __uint_as_float(v[e + 3]))
+                           : "memory");
+            else
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (e + i < n) atomicAdd(q + e + i, p.alpha * __uint_as_float(v[e + i]));
+          }
+        } else {
+          float* q = p.outf + o;
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            if (e + 4 <= n)
+              *reinterpret_cast<float4*>(q + e) =
+                  make_float4(p.alpha * __uint_as_float(v[e]), p.alpha * __uint_as_float(v[e + 1]),
+                              p.alpha * __uint_as_float(v[e + 2]), p.alpha * __uint_as_float(v[e + 3]));
+            else
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (e + i < n) q[e + i] = p.alpha * __uint_as_float(v[e + i]);
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+      __syncwarp();
+      if (lane == 0) arrive_rank0(tempty0 + 8 * acc);
+    }
+  }
+  __syncwarp();
+  if (!__syncthreads_and(ok) && threadIdx.x == 0) atomicExch(&g_tc_error, 1);
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+  cluster_sync();  // neither CTA leaves while the other may still signal it
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(2 * pair::BN));
+  cluster_sync();
+}
+
+// Takes what the plain single-CTA kernel takes, with an output and no epilogue terms, where
+// 256-row tiles waste little: an even number of 128-row tiles, or at least eight.
+bool pair_eligible(const GemmP& p) {
+  const long long rows = ceil_div(p.M, 128);
+  const uintptr_t out = reinterpret_cast<uintptr_t>(p.outh ? (const void*)p.outh : (const void*)p.outf);
+  return p.batch == 1 && (rows % 2 == 0 || rows >= 8) && !(p.outh && p.outf) && !(p.outh && p.atomic) && !p.cadd &&
+         !p.cadd_h && !p.bias_m && !p.bias_n && !p.pre && p.act == 0 && (out & 15u) == 0u &&
+         p.ldc % (p.outh ? 8 : 4) == 0 && (p.splitk - 1) * ceil_div(ceil_div(p.K, 64), p.splitk) < ceil_div(p.K, 64);
+}
+
+// 1: launched; 0: not applicable here (caller uses another kernel); <0: error status.
+int launch_gemm_pair(const GemmP& p, cudaStream_t st) {
+  alignas(64) CUtensorMap ma, mb;
+  if (!make_map(&ma, p.A, p.M, p.K, p.lda, 128) || !make_map(&mb, p.B, p.N, p.K, p.ldb, 128)) return 0;
+  // Pairs that are resident at once (a GPC with an odd number of SMs leaves one out); more
+  // would wait for a whole pass of the persistent ones. Asked once per device.
+  static std::atomic<int> resident[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return fail(BZ_ERR_CUDA, "bz_gemm_bf16: no current device");
+  if (dev >= 64) return 0;
+  int slots = resident[dev].load();
+  if (slots == 0) {
+    if (cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM) != cudaSuccess)
+      return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the pair kernel's shared memory");
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(148);
+    cfg.blockDim = dim3(pair::THREADS);
+    cfg.dynamicSmemBytes = pair::SMEM;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&slots, gemm_pair_kernel, &cfg) != cudaSuccess)
+      return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot query the pair kernel's residency");
+    if (slots < 1) return 0;
+    resident[dev].store(slots);
+  }
+  const int m_tiles = (int)ceil_div(p.M, pair::BM), n_tiles = (int)ceil_div(p.N, pair::BN);
+  const long long total = (long long)m_tiles * n_tiles * p.splitk;
+  if (total > (1LL << 30)) return 0;
+  const int pairs = (int)(total < slots ? total : slots);
+  gemm_pair_kernel<<<2 * pairs, pair::THREADS, pair::SMEM, st>>>(ma, mb, p, m_tiles, n_tiles);
+  const int rc = check_launch("bz_gemm_bf16");
+  return rc == BZ_OK ? 1 : rc;
+}
+
 bool tc_eligible(const GemmP& p) {
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0u; };
   return !p.ta && p.tb && p.M >= 128 && p.N >= 256 && p.K >= 64 && p.lda % 8 == 0 && p.ldb % 8 == 0 &&
@@ -763,18 +1074,6 @@ __device__ __forceinline__ uint64_t tc_sdesc_sw128_mn(uint32_t saddr, uint32_t l
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)2 << 61;
   return d;
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
 template <int KC, int MC>
@@ -1458,6 +1757,10 @@ extern "C" int bz_gemm_bf16(const bz_gemm* g, void* stream) {
   p.withhold = 0;
   cudaStream_t st = bz::as_stream(stream);
   if (g->engine == 0 && bz::tc_eligible(p)) {
+    if (bz::pair_eligible(p)) {
+      const int t = bz::launch_gemm_pair(p, st);
+      if (t != 0) return t > 0 ? BZ_OK : t;
+    }
     const int t = bz::launch_gemm_tma(p, st);
     if (t != 0) return t > 0 ? BZ_OK : t;
     return bz::launch_gemm_tc(p, st);

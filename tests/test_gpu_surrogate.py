@@ -382,6 +382,39 @@ def test_tma_gemm_plain_bf16_output(bz):
     assert rel(outh.float(), want) <= 8e-3
 
 
+@pytest.mark.parametrize("out", ["f32", "bf16", "atomic"])
+@pytest.mark.parametrize("M,N,K,splitk", [(256, 256, 64, 1), (512, 260, 72, 1), (1100, 520, 200, 3), (2304, 768, 1032, 2),
+                                          (256, 8192, 128, 1)])
+def test_pair_gemm_matches_f32_matmul(bz, M, N, K, splitk, out):
+    """CTA-pair GEMM: one tile, several per pair, ragged rows, columns and K, K splits.
+    float32 accumulation order only: 1e-5; bf16 outputs 8e-3."""
+    from beamz_b200 import _native as nat
+
+    if splitk > 1 and out != "atomic":
+        pytest.skip("split-K accumulates atomically")
+    g = torch.Generator().manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    B = torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+    ld = (N + 7) // 8 * 8
+    base = torch.randn(M, ld, generator=g).cuda()
+    o = base.clone() if out != "bf16" else base.to(torch.bfloat16)
+    p = nat.Gemm()
+    p.M, p.N, p.K, p.batch, p.splitk, p.ta, p.tb, p.atomic = M, N, K, 1, splitk, 0, 1, int(out == "atomic")
+    p.A, p.lda, p.B, p.ldb, p.alpha, p.ldc = A.data_ptr(), K, B.data_ptr(), K, 0.5, ld
+    if out == "bf16":
+        p.outh = o.data_ptr()
+    else:
+        p.outf = o.data_ptr()
+    nat.gemm(p, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert nat.gemm_error(reset=True) == 0
+    want = 0.5 * (A.float() @ B.float().t())
+    if out == "atomic":
+        want = want + base[:, :N]
+    assert rel(o[:, :N].float(), want) <= (8e-3 if out == "bf16" else 1e-5)
+    assert torch.equal(o[:, N:].float(), base[:, N:].to(o.dtype).float())  # padding columns stay
+
+
 def test_fno_with_tcgen05_spectral_gemms_matches_oracle(bz):
     """n = 64, 8 modes, width 32, batch 8: the DFT GEMMs (M = 256, N = 256, K = 4096)
     and their inverses run on the tcgen05 kernel."""
