@@ -415,6 +415,27 @@ def test_pair_gemm_matches_f32_matmul(bz, M, N, K, splitk, out):
     assert torch.equal(o[:, N:].float(), base[:, N:].to(o.dtype).float())  # padding columns stay
 
 
+@pytest.mark.parametrize("K,N,batch", [(3, 14400, 2), (1, 32, 1), (16, 72, 3), (7, 1000, 5)])
+def test_lift_layer_matches_general_kernel(bz, K, N, batch):
+    """The 32-channel lift kernel against the general kernel (engine 1), bit for bit."""
+    from beamz_b200 import _native as nat
+
+    g = torch.Generator().manual_seed(K * N)
+    W = torch.randn(32, K, generator=g).to(torch.bfloat16).cuda()
+    X = torch.randn(batch, K, N, generator=g).to(torch.bfloat16).cuda()
+    bias = torch.randn(32, generator=g).cuda()
+    outs = []
+    for engine in (1, 0):
+        o = torch.empty(batch, 32, N, dtype=torch.bfloat16, device="cuda")
+        p = nat.Gemm()
+        p.M, p.N, p.K, p.batch, p.splitk, p.engine, p.alpha = 32, N, K, batch, 1, engine, 1.0
+        p.A, p.lda, p.B, p.ldb, p.sb = W.data_ptr(), K, X.data_ptr(), N, K * N
+        p.bias_m, p.outh, p.ldc, p.sc = bias.data_ptr(), o.data_ptr(), N, 32 * N
+        nat.gemm(p, torch.cuda.current_stream().cuda_stream)
+        outs.append(o)
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_fno_with_tcgen05_spectral_gemms_matches_oracle(bz):
     """n = 64, 8 modes, width 32, batch 8: the DFT GEMMs (M = 256, N = 256, K = 4096)
     and their inverses run on the tcgen05 kernel."""
