@@ -166,7 +166,8 @@ class FNO2d:
             S = torch.empty((B * C, P), dtype=BF16, device=self.dev)
             self._gemm(B * C, P, 2 * self.K, O, 2 * self.K, self.GT, 2 * self.K, tb=1, outh=S)
             act = 1 if l < self.L else 0
-            pre = torch.empty((B, C, P), dtype=BF16, device=self.dev) if act else None
+            # the pre-activation is only read by the backward pass
+            pre = torch.empty((B, C, P), dtype=BF16, device=self.dev) if act and keep else None
             Vn = torch.empty((B, C, P), dtype=BF16, device=self.dev)
             self._gemm(C, P, C, p[f"W{l}"].h, C, V, P, batch=B, sb=C * P, outh=Vn, sc=C * P, cadd_h=S, ldadd=P,
                        sadd=C * P, bias_m=p[f"b{l}"].w, act=act, pre=pre)
@@ -176,7 +177,7 @@ class FNO2d:
             acts["V"].append(Vn)
             V = Vn
         Hh = torch.empty((B, Hd, P), dtype=BF16, device=self.dev)
-        preh = torch.empty_like(Hh)
+        preh = torch.empty_like(Hh) if keep else None
         self._gemm(Hd, P, C, p["Q1"].h, C, V, P, batch=B, sb=C * P, outh=Hh, sc=Hd * P, bias_m=p["q1"].w, act=1,
                    pre=preh)
         pooled = torch.empty((B, Hd), dtype=torch.float32, device=self.dev)
