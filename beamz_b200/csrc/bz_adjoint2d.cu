@@ -238,7 +238,7 @@ __device__ __forceinline__ void adj_run(const AdjArgs<T>& a, int d, int k, int k
 }
 
 template <typename T, int TS, int R, int NW, int MINB>
-__global__ void __launch_bounds__(32 * NW, MINB) adjoint2d_tb_kernel(AdjArgs<T> a, bool vec, long long step0) {
+__global__ void __launch_bounds__(32 * NW, MINB) adjoint2d_tb_kernel(AdjArgs<T> a, int ahead, bool vec, long long step0) {
   typedef typename PairOf<T>::type V;
   typedef AdjSmem<T, TS, R, NW> S;
   constexpr int TH = S::TH, HX = TS + 1, OW = TBW - 2 * HX, OH = TH - 2 * TS, NT = 32 * NW;
@@ -293,6 +293,16 @@ __global__ void __launch_bounds__(32 * NW, MINB) adjoint2d_tb_kernel(AdjArgs<T> 
       cc[i] = ld_pair(a.ce + mb + r, in0 && iny, in1 && iny);
     }
     hyu = ld_pair(a.hy_in + fb - pitch, in0 && yb >= 1 && yb < ny, in1 && yb >= 1 && yb < ny);
+  }
+  if (ahead > 0) {  // the tile that a block of the next wave will load
+    const long long next = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x + ahead;
+    const int bz = (int)(next / ((long long)gridDim.x * gridDim.y));
+    if (bz < (int)gridDim.z) {
+      const int rem = (int)(next - (long long)bz * gridDim.x * gridDim.y), by = rem / (int)gridDim.x, bx = rem - by * (int)gridDim.x;
+      const long long pf = (long long)bz * a.plane, pm = a.n_mat > 1 ? pf : 0LL;
+      const T* const arr[5] = {a.e_in + pf, a.hx_in + pf, a.hy_in + pf, a.ce + pm, a.loss + pm};
+      prefetch_tile<T, TH, NW>(arr, bx * OW - HX, by * OH - TS, ny, pitch, w, lane);
+    }
   }
   __syncthreads();  // the pool's counter is set
 
@@ -602,7 +612,9 @@ int launch_adj_tb(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops
   const bool vec = bits % (2 * sizeof(T)) == 0;
   dim3 grid((unsigned)ceil_div(g->nx, TBW - 2 * (TS + 1)), (unsigned)ceil_div(g->ny, NW * R - 2 * TS),
             (unsigned)g->n_designs);
-  kernel<<<grid, 32 * NW, SMEM, st>>>(a, vec, (long long)step);
+  const int ahead = prefetch_distance((long long)sizeof(T) * a.plane * (6LL * g->n_designs + 2LL * g->n_mat),
+                                      (long long)grid.x * grid.y * grid.z);
+  kernel<<<grid, 32 * NW, SMEM, st>>>(a, ahead, vec, (long long)step);
   return check_launch("bz_adjoint_step2d_multi");
 }
 

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) step2d_tb_kernel(
     T* __restrict__ ez_out, T* __restrict__ hx_out, T* __restrict__ hy_out,
     const T* __restrict__ ce, const T* __restrict__ loss, double* __restrict__ pwr, Geo2D<T> g, Ops2D<T> o,
     int n_comp, int plane0,
-    int n_planes, bool vec, long long step_base, const long long* __restrict__ d_step) {
+    int n_planes, int ahead, bool vec, long long step_base, const long long* __restrict__ d_step) {
   typedef typename PairOf<T>::type V;
   typedef TbSmem<T, TS, R, NW> S;
   constexpr int TH = S::TH, HX = TS + 1;
@@ -393,6 +393,17 @@ __global__ void __launch_bounds__(32 * NW, MINB) step2d_tb_kernel(
       cc[i] = ld_pair(ce + mb + r, in0 && iny, in1 && iny);
     }
     hyu = ld_pair(hy_in + fb - pitch, in0 && yb >= 1 && yb < ny, in1 && yb >= 1 && yb < ny);
+  }
+  if (ahead > 0) {  // the tile that a block of the next wave will load
+    const long long next = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x + ahead;
+    const int bz = (int)(next / ((long long)gridDim.x * gridDim.y));
+    if (bz < (int)gridDim.z) {
+      const int rem = (int)(next - (long long)bz * gridDim.x * gridDim.y), by = rem / (int)gridDim.x, bx = rem - by * (int)gridDim.x;
+      const long long pf = (long long)(plane0 + bz) * g.plane;
+      const long long pm = (g.n_mat > 1 ? (long long)((plane0 + bz) / n_comp) : 0LL) * g.plane;
+      const T* const arr[5] = {ez_in + pf, hx_in + pf, hy_in + pf, ce + pm, loss + pm};
+      prefetch_tile<T, TH, NW>(arr, bx * OW - HX, by * OH - TS, ny, pitch, w, lane);
+    }
   }
   __syncthreads();  // the pools' counters are set
 
@@ -772,13 +783,15 @@ int launch_tb(const bz_grid2d* gd, const bz_fields2d* f, const bz_source_ops* s,
   const bool vec = bits % (2 * sizeof(T)) == 0;  // pairs start at even columns and the pitch is even
   const int src = (int)(step & 1);
   const int n_planes = gd->n_designs * gd->n_comp;
+  const int ahead = prefetch_distance((long long)sizeof(T) * g.plane * (6LL * n_planes + 2LL * gd->n_mat),
+                                      ceil_div(gd->nx, OW) * ceil_div(gd->ny, OH) * (long long)n_planes);
   for (int p0 = 0; p0 < n_planes; p0 += 65535) {  // the z extent of a grid is at most 65535
     dim3 grid((unsigned)ceil_div(gd->nx, OW), (unsigned)ceil_div(gd->ny, OH),
               (unsigned)(n_planes - p0 < 65535 ? n_planes - p0 : 65535));
     kernel<<<grid, 32 * NW, SMEM, st>>>(
         (const T*)f->ez[src], (const T*)f->hx[src], (const T*)f->hy[src], (T*)f->ez[src ^ 1], (T*)f->hx[src ^ 1],
         (T*)f->hy[src ^ 1], (const T*)f->ce, (const T*)f->loss, f->power, g, o, gd->n_comp, p0, n_planes,
-        vec,
+        ahead, vec,
         (long long)step, (const long long*)d_step);
   }
   return check_launch("bz_step2d_multi");

@@ -86,4 +86,28 @@ __device__ __forceinline__ unsigned scan_ops(const int* __restrict__ cells, int 
   return __reduce_or_sync(FULL, rows);
 }
 
+// Asks for the tile that starts at column X and row Y of five arrays to be brought into L2:
+// the lanes of a warp take the arrays' 128-byte lines of one row (pitch and rows are
+// multiples of a line).
+template <typename T, int TH, int NW>
+__device__ __forceinline__ void prefetch_tile(const T* const (&arr)[5], int X, int Y, int ny, int pitch, int warp, int lane) {
+  constexpr int PER = 128 / (int)sizeof(T), LINES = TBW / PER + 1;  // a tile row starts anywhere in a line
+  static_assert(5 * LINES <= 32, "one lane a line");
+  const int a = lane / LINES, col = (max(X, 0) & ~(PER - 1)) + (lane - a * LINES) * PER;
+  if (a >= 5 || col >= pitch) return;
+  const T* p = a == 0 ? arr[0] : a == 1 ? arr[1] : a == 2 ? arr[2] : a == 3 ? arr[3] : arr[4];
+  for (int r = warp; r < TH; r += NW) {
+    const int y = Y + r;
+    if (y >= 0 && y < ny) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (long long)y * pitch + col));
+  }
+}
+
+// Blocks between a tile and the one to prefetch: the blocks an SM runs side by side times
+// the SMs, where the arrays do not stay in L2 from one launch to the next (and there is
+// more than one such wave); 0: no prefetch.
+inline int prefetch_distance(long long bytes, long long blocks) {
+  constexpr long long WAVE = 2 * 148;
+  return bytes > (100LL << 20) && blocks > 2 * WAVE ? (int)WAVE : 0;
+}
+
 }  // namespace bz
