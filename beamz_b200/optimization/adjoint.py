@@ -236,7 +236,7 @@ class AdjointFDTD2D:
         ops.sig, ops.signals = t(sig, torch.int32).data_ptr(), t(signals, dt_).data_ptr()
         ops.weight_stride = len(cell)
         shape = (self.B, self.ny, eng.pitch)
-        st = torch.cuda.current_stream().cuda_stream
+        st = nat.current_stream()
         E = [torch.zeros(shape, dtype=dt_, device=dev) for _ in range(2)]
         HX = [torch.zeros_like(E[0]) for _ in range(2)]
         HY = [torch.zeros_like(E[0]) for _ in range(2)]

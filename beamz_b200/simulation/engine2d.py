@@ -197,7 +197,7 @@ class Engine2D:
     # ---- stepping -------------------------------------------------------------
     @staticmethod
     def _stream() -> int:
-        return torch.cuda.current_stream().cuda_stream
+        return nat.current_stream()
 
     def _fields(self) -> nat.Fields2D:
         # The copy holding the current fields is always (step_index & 1): every
@@ -387,6 +387,8 @@ class Engine2D:
                 self.n_step_launches += 1
                 self.step_index += k
                 n -= k
+                if self.step_index % self.chunk == 0:  # the grouping of the DFT sums that chunks give
+                    self._fold()
                 continue
             self.step_once()
             n -= 1

@@ -93,7 +93,7 @@ class Engine3D:
 
     @staticmethod
     def _stream():
-        return torch.cuda.current_stream().cuda_stream
+        return nat.current_stream()
 
     def _kept(self, t):
         self._keep.append(t)

@@ -29,7 +29,7 @@ class DivergenceGuard:
 
     def check(self, field: torch.Tensor, bz_dtype: int, step: int) -> None:
         nat.field_check(field.data_ptr(), bz_dtype, field.numel(), self.limit, step, self.status.data_ptr(),
-                        torch.cuda.current_stream().cuda_stream)
+                        nat.current_stream())
         self.launches += 1
 
     def maybe_check(self, field: torch.Tensor, bz_dtype: int, step: int) -> None:

@@ -98,7 +98,7 @@ class FNO2d:
     # ---- kernel helpers ---------------------------------------------------------------
     @staticmethod
     def _stream() -> int:
-        return torch.cuda.current_stream().cuda_stream
+        return nat.current_stream()
 
     def _gemm(self, M, N, K, A, lda, B, ldb, *, batch=1, sa=0, sb=0, ta=0, tb=0, outf=None, outh=None, ldc=None,
               sc=0, cadd=None, cadd_h=None, ldadd=0, sadd=0, bias_m=None, bias_n=None, act=0, pre=None, atomic=0,
@@ -305,7 +305,7 @@ def bench_mixing(reps: int = 20) -> list:
     per second (activations read, f32 term read, pre-activation and output written)."""
     dev = torch.device("cuda")
     B, P = 64, 120 * 120
-    st = torch.cuda.current_stream().cuda_stream
+    st = nat.current_stream()
     rows = []
     # (M, K, ta, fused): the forward layer (f32 term, bias, pre-activation, GELU), the head's
     # first layer, the head's transposed layer in the backward, a transposed layer with
