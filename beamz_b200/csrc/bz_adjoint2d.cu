@@ -590,12 +590,10 @@ int launch_adj(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops* o
   return check_launch("bz_adjoint_step2d");
 }
 
-template <typename T, int TS>
-int launch_adj_tb(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops* ops, int64_t step, int32_t phase,
-                  cudaStream_t st) {
-  // float: 64 x 64 tiles, two blocks an SM up to five steps; double: 64 x 32
-  constexpr int R = sizeof(T) == 4 ? 8 : 2, NW = sizeof(T) == 4 ? 8 : 16;
-  constexpr int SMEM = AdjSmem<T, TS, R, NW>::BYTES, MINB = sizeof(T) == 4 ? 2 : 1;
+template <typename T, int TS, int R, int NW, int MINB>
+int launch_adj_tile(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops* ops, int64_t step, int32_t phase,
+                    cudaStream_t st) {
+  constexpr int SMEM = AdjSmem<T, TS, R, NW>::BYTES;
   const auto kernel = adjoint2d_tb_kernel<T, TS, R, NW, MINB>;
   const AdjArgs<T> a = adj_args<T>(g, s, ops, phase);
   int dev = 0;
@@ -616,6 +614,19 @@ int launch_adj_tb(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops
                                       (long long)grid.x * grid.y * grid.z);
   kernel<<<grid, 32 * NW, SMEM, st>>>(a, ahead, vec, (long long)step);
   return check_launch("bz_adjoint_step2d_multi");
+}
+
+// float: 64 x 64 tiles, two blocks an SM up to five steps; where those leave SMs idle, 64 x
+// 32 tiles of two rows a warp, whose sub-steps are shorter (300 x 200 cells, one design,
+// nine steps a launch: 800 reverse steps 3.6 -> 2.2 ms). double: 64 x 32.
+template <typename T, int TS>
+int launch_adj_tb(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_ops* ops, int64_t step, int32_t phase,
+                  cudaStream_t st) {
+  if constexpr (sizeof(T) == 4) {
+    const long long tiles = ceil_div(g->nx, TBW - 2 * (TS + 1)) * ceil_div(g->ny, 64 - 2 * TS) * (long long)g->n_designs;
+    if (tiles >= 148) return launch_adj_tile<T, TS, 8, 8, 2>(g, s, ops, step, phase, st);
+  }
+  return launch_adj_tile<T, TS, 2, 16, 1>(g, s, ops, step, phase, st);
 }
 
 }  // namespace

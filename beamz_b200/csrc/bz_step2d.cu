@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) step2d_tb_kernel(
       const bool iny = y >= 0 && y < ny, inh = y >= 0 && y < ny - 1, inty = y >= 1 && y <= ny - 2;
       const bool i0 = inty && xa >= 1 && xa <= nx - 2, i1 = inty && xa + 1 >= 1 && xa + 1 <= nx - 2;
       T fh0, fh1, cx0, cx1, cy0, cy1;
-      h_coeffs(lo2(ls[i]), g.chx, g.chy, fh0, cx0, cy0);  // divisions: rows free of loss skip them
+      h_coeffs(lo2(ls[i]), g.chx, g.chy, fh0, cx0, cy0);
       h_coeffs(hi2(ls[i]), g.chx, g.chy, fh1, cx1, cy1);
       const T fe0 = i0 ? sub_rn(T(1), mul_rn(mul_rn(lo2(ls[i]), lo2(cc[i])), g.inv_kd2)) : T(1);
       const T fe1 = i1 ? sub_rn(T(1), mul_rn(mul_rn(hi2(ls[i]), hi2(cc[i])), g.inv_kd2)) : T(1);

@@ -219,11 +219,14 @@ def test_backward_without_checkpoints_or_history_is_an_error(bz):
 
 
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("fp32", 2e-5)])
-@pytest.mark.parametrize("ny,nx,pml,box", [(150, 200, 8, (50, 60, 37, 61)), (131, 173, 6, (7, 9, 30, 41)), (40, 66, 0, (3, 4, 9, 7))])
-def test_reverse_tiles_match_single_steps(bz, ny, nx, pml, box, precision, tol):
+@pytest.mark.parametrize("ny,nx,pml,box,designs", [(150, 200, 8, (50, 60, 37, 61), 2), (150, 200, 8, (50, 60, 37, 61), 13),
+                                                   (131, 173, 6, (7, 9, 30, 41), 2), (131, 173, 6, (7, 9, 30, 41), 14),
+                                                   (40, 66, 0, (3, 4, 9, 7), 2)])
+def test_reverse_tiles_match_single_steps(bz, ny, nx, pml, box, designs, precision, tol):
     """Gradients of every reverse block length against single reverse steps: tiles clear
     of loss and edges, a box next to the absorber (tiles that need factors and gradient
-    history at once), a grid without loss smaller than a tile. float64 agrees to rounding
+    history at once), a grid without loss smaller than a tile; few designs (small float
+    tiles) and enough of them for the large ones. float64 agrees to rounding
     of the reassociated sums, float32 within the stepping tolerance."""
     from beamz_b200.optimization.adjoint import AdjointFDTD2D
 
@@ -238,11 +241,11 @@ def test_reverse_tiles_match_single_steps(bz, ny, nx, pml, box, precision, tol):
     sig = np.sin(2 * np.pi * 1.9e14 * np.arange(n) * dt + 0.5)
     src = bz.GaussianSource(position=((x0 + w + 4) * dx, (y0 + h // 2) * dx), width=dx, signal=sig)
     mon = bz.Monitor(start=((x0 + w + 9) * dx, y0 * dx), end=((x0 + w + 9) * dx, (y0 + h) * dx))
-    er = 2.0 + 10.0 * rng.random((2, h, w))
+    er = 2.0 + 10.0 * rng.random((designs, h, w))
     grads = {}
     for k in (1, 3, 5, 7, 9):
         p = AdjointFDTD2D(1.0 + 11.0 * np.random.default_rng(3).random((ny, nx)), sigma, dx, dt, n, [src], mon,
-                          np.ones(h + 1, dtype=complex), [1.9e14, 2.1e14], box, n_designs=2, precision=precision)
+                          np.ones(h + 1, dtype=complex), [1.9e14, 2.1e14], box, n_designs=designs, precision=precision)
         p._adj_block = k
         grads[k] = p.value_and_grad(er)[1]
     assert np.abs(grads[1]).max() > 0
