@@ -144,6 +144,7 @@ _spec = _sig("bz_spectral_mix", C.c_int, [vp, vp, vp, i32, i32, i32, i32, vp])
 _spec_bwd = _sig("bz_spectral_mix_bwd", C.c_int, [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp])
 _gelu_bwd = _sig("bz_gelu_bwd", C.c_int, [vp, vp, vp, i64, vp])
 _row_mean = _sig("bz_row_mean", C.c_int, [vp, vp, i64, i32, C.c_float, vp])
+_mix_mean = _sig("bz_mix_mean", C.c_int, [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, C.c_float, vp])
 _row_bcast = _sig("bz_row_broadcast", C.c_int, [vp, vp, i64, i32, C.c_float, vp])
 _chan_sum = _sig("bz_chan_sum", C.c_int, [vp, vp, i32, i32, i32, vp])
 _adam = _sig("bz_adam", C.c_int, [vp, vp, vp, vp, vp, i64, C.c_float, C.c_float, C.c_float, C.c_float, i32,
@@ -157,7 +158,7 @@ _field_check = _sig("bz_field_check", C.c_int, [vp, i32, i64, f64, i64, vp, vp])
 EXPORTED = ["bz_version", "bz_last_error", "bz_step2d", "bz_step2d_multi", "bz_step2d_multi_power", "bz_dft_fold", "bz_step2d_dft_static", "bz_advance_step",
             "bz_adjoint_step2d", "bz_adjoint_step2d_multi", "bz_step3d", "bz_cell_ops", "bz_gather", "bz_power3d", "bz_dft_fold_q", "bz_rasterize3d", "bz_prepare_coeffs", "bz_update_h2d",
             "bz_update_e2d", "bz_rasterize2d", "bz_gemm_bf16", "bz_spectral_mix", "bz_spectral_mix_bwd", "bz_gelu_bwd",
-            "bz_row_mean", "bz_row_broadcast", "bz_chan_sum", "bz_adam", "bz_to_bf16", "bz_gemm_error",
+            "bz_row_mean", "bz_mix_mean", "bz_row_broadcast", "bz_chan_sum", "bz_adam", "bz_to_bf16", "bz_gemm_error",
             "bz_gemm_wait_selftest", "bz_field_check"]
 
 
@@ -279,6 +280,10 @@ def spectral_mix_bwd(dO, U, W, dU, dW, B, ci, co, n_modes, stream) -> None:
 
 def gelu_bwd(dy, pre, dx, n, stream) -> None:
     check(_gelu_bwd(dy, pre, dx, n, stream))
+
+
+def mix_mean(W, X, bias, pre, part, mean, batch, M, K, P, scale, stream) -> None:
+    check(_mix_mean(W, X, bias, pre, part, mean, batch, M, K, P, scale, stream))
 
 
 def row_mean(x, out, rows, P, scale, stream) -> None:

@@ -1093,6 +1093,13 @@ struct MixCfg {
 // arithmetic (branches that each wait for their predicate): at 256 designs of 14400 pixels
 // 32 -> 32 channels with an added term 253 -> 147 us, 32 -> 64 534 -> 179 us, both with
 // GELU and no pre-activation.
+// Bit 2 (with bit 1): the result itself is not stored, only each channel's sum over the
+// tile's 128 pixels, of the values rounded to bf16 as they would be stored, in
+// outf[tile][channel] (tiles of a design in order). A warp folds its 32 pixels x 32
+// channels so that each lane ends with one channel (31 shuffles for 32 sums), the four
+// warps meet in shared memory. 256 designs, 32 -> 64 channels: 179 us and 126 us for the
+// means of the stored values -> 193 + 7 us, about half of it the tanh unit (64 a pixel at 16
+// a clock and SM).
 template <int KC, int MC, int EPI>
 __global__ void __launch_bounds__(mix::THREADS) mix_tc_kernel(const __grid_constant__ CUtensorMap tmX, GemmP p,
                                                              int n_tiles, int tiles_n) {
@@ -1122,7 +1129,9 @@ __global__ void __launch_bounds__(mix::THREADS) mix_tc_kernel(const __grid_const
     const bf16 w = p.ta ? p.A[(long long)k * p.lda + m] : p.A[(long long)m * p.lda + k];
     *reinterpret_cast<bf16*>(smem + C::W_OFF + (k >> 3) * C::LBO_W + (m >> 3) * 128 + (m & 7) * 16 + (k & 7) * 2) = w;
   }
+  constexpr bool POOL = EPI >= 0 && (EPI & 4) != 0;
   __shared__ float s_bias[MC];
+  __shared__ float s_part[POOL ? 4 : 1][POOL ? MC : 1];
   for (int i = tid; i < MC; i += mix::THREADS) s_bias[i] = p.bias_m ? p.bias_m[i] : 0.f;
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
@@ -1174,7 +1183,8 @@ __global__ void __launch_bounds__(mix::THREADS) mix_tc_kernel(const __grid_const
     float add[MC];
 #pragma unroll
     for (int e = 0; e < MC; ++e) add[e] = 0.f;
-    if (p.cadd && live) {
+    if (POOL) {  // takes no added term
+    } else if (p.cadd && live) {
       const float* q = p.cadd + (long long)b * p.sadd + n;
 #pragma unroll
       for (int e = 0; e < MC; ++e) add[e] = __ldg(q + (long long)e * p.ldadd);
@@ -1198,6 +1208,32 @@ __global__ void __launch_bounds__(mix::THREADS) mix_tc_kernel(const __grid_const
     for (int c0 = 0; c0 < MC; c0 += 32) {
       uint32_t v[32];
       tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)((j & 1) * C::NCOL + c0), v);
+      if constexpr (POOL) {
+        float y[32];
+        const unsigned mask = live ? 0xffffffffu : 0u;  // not a select: that became a branch around each GELU
+        bf16* pq = p.pre + (long long)b * p.spre + (long long)c0 * p.ldpre + n;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          y[e] = p.alpha * __uint_as_float(v[e]) + s_bias[c0 + e];
+          if constexpr ((EPI & 1) != 0) {
+            if (live) *pq = __float2bfloat16_rn(y[e]);
+            pq += p.ldpre;
+          }
+          const float h = __bfloat162float(__float2bfloat16_rn(gelu_bf16out(y[e])));
+          y[e] = __uint_as_float(__float_as_uint(h) & mask);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {  // lanes with bit o keep the upper half of the channels
+          const bool up = (lane & o) != 0;
+#pragma unroll
+          for (int e = 0; e < o; ++e) {
+            const float give = up ? y[e] : y[e + o], keep = up ? y[e + o] : y[e];
+            y[e] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        s_part[warp][c0 + lane] = y[0];
+        continue;
+      }
       if (!live) continue;
       // output rows walked by pointer increments (one 64-bit add per element and array)
       const long long o0 = (long long)b * p.sc + (long long)c0 * p.ldc + n;
@@ -1240,6 +1276,8 @@ __global__ void __launch_bounds__(mix::THREADS) mix_tc_kernel(const __grid_const
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
     __syncthreads();  // accumulator j & 1 read out before tile j + 2's MMAs overwrite it
+    if (POOL && tid < MC)  // the next tile's sums come after its own block barrier
+      p.outf[(long long)t * MC + tid] = (s_part[0][tid] + s_part[1][tid]) + (s_part[2][tid] + s_part[3][tid]);
   }
   if (tid == 0) {
     if (!ok && mmas > 0)  // let issued MMAs drain before the TMEM goes
@@ -1306,10 +1344,32 @@ int launch_mix_kc_mc(const GemmP& p, cudaStream_t st) {
   return p.pre ? launch_mix_epi<KC, MC, 1>(p, st) : launch_mix_epi<KC, MC, 0>(p, st);
 }
 
+template <int KC, int MC>
+int launch_mix_mean(const GemmP& p, cudaStream_t st) {
+  return p.pre ? launch_mix_epi<KC, MC, 7>(p, st) : launch_mix_epi<KC, MC, 6>(p, st);
+}
+
 // 1: launched; 0: not applicable (caller uses another kernel); <0: error status.
 int launch_mix(const GemmP& p, cudaStream_t st) {
   if (p.K == 32) return p.M == 32 ? launch_mix_kc_mc<32, 32>(p, st) : launch_mix_kc_mc<32, 64>(p, st);
   return p.M == 32 ? launch_mix_kc_mc<64, 32>(p, st) : launch_mix_kc_mc<64, 64>(p, st);
+}
+
+// mean[b][c] = scale * sum_t part[b][t][c]: one block per design, 256 / M tiles at a time.
+__global__ void __launch_bounds__(256) tile_mean_kernel(const float* __restrict__ part, float* __restrict__ mean,
+                                                        int M, int tiles, float scale) {
+  __shared__ float s[256];
+  const int c = threadIdx.x % M, g = threadIdx.x / M, G = 256 / M;
+  const float* q = part + (long long)blockIdx.x * tiles * M + c;
+  float a = 0.f;
+#pragma unroll 4
+  for (int t = g; t < tiles; t += G) a += q[(long long)t * M];
+  s[threadIdx.x] = a;
+  __syncthreads();
+  if (g == 0) {
+    for (int i = 1; i < G; ++i) a += s[i * M + c];
+    mean[(long long)blockIdx.x * M + c] = a * scale;
+  }
 }
 
 // ---- lift layer: C[b] = W (32 x K) @ X[b] (K x N) + bias, K <= 16, bf16 out -------------
@@ -1887,6 +1947,31 @@ extern "C" int bz_gemm_bf16(const bz_gemm* g, void* stream) {
   if (g->N <= 32) return bz::launch_gemm<128, 32, 4, 1>(p, st);
   if (g->M <= 32) return bz::launch_gemm<32, 128, 1, 4>(p, st);
   return bz::launch_gemm<128, 128, 2, 4>(p, st);
+}
+
+extern "C" int bz_mix_mean(const void* W, const void* X, const float* bias, void* pre, float* part, float* mean,
+                           int32_t batch, int32_t M, int32_t K, int32_t P, float scale, void* stream) {
+  BZ_REQUIRE(W && X && part && mean, "bz_mix_mean: NULL buffer");
+  BZ_REQUIRE((M == 32 || M == 64) && (K == 32 || K == 64), "bz_mix_mean: M=%d K=%d, 32 or 64 each", M, K);
+  BZ_REQUIRE(P >= 64 && P % 8 == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0u,
+             "bz_mix_mean: P=%d, a multiple of 8 from 64 on, X on 16 bytes", P);
+  BZ_REQUIRE(batch >= 1 && batch <= 65535, "bz_mix_mean: batch %d", batch);
+  bz::GemmP p = {};
+  p.M = M; p.N = P; p.K = K; p.batch = batch; p.splitk = 1; p.act = 1;
+  p.A = (const bz::bf16*)W; p.lda = K;
+  p.B = (const bz::bf16*)X; p.ldb = P; p.sb = (long long)K * P;
+  p.alpha = 1.0f;
+  p.bias_m = bias;
+  p.outf = part;
+  p.pre = (bz::bf16*)pre; p.ldpre = P; p.spre = (long long)M * P;
+  p.wait_limit = bz::tc::WAIT_LIMIT;
+  cudaStream_t st = bz::as_stream(stream);
+  const int t = K == 32 ? (M == 32 ? bz::launch_mix_mean<32, 32>(p, st) : bz::launch_mix_mean<32, 64>(p, st))
+                        : (M == 32 ? bz::launch_mix_mean<64, 32>(p, st) : bz::launch_mix_mean<64, 64>(p, st));
+  if (t < 0) return t;
+  if (t == 0) return bz::fail(BZ_ERR_CUDA, "bz_mix_mean: no tensor map for X");
+  bz::tile_mean_kernel<<<batch, 256, 0, st>>>(part, mean, M, (int)bz::ceil_div(P, bz::mix::TP), scale);
+  return bz::check_launch("bz_mix_mean");
 }
 
 extern "C" int bz_gemm_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, void* stream) {

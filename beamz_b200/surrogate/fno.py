@@ -176,12 +176,19 @@ class FNO2d:
             acts["pre"].append(pre)
             acts["V"].append(Vn)
             V = Vn
-        Hh = torch.empty((B, Hd, P), dtype=BF16, device=self.dev)
-        preh = torch.empty_like(Hh) if keep else None
-        self._gemm(Hd, P, C, p["Q1"].h, C, V, P, batch=B, sb=C * P, outh=Hh, sc=Hd * P, bias_m=p["q1"].w, act=1,
-                   pre=preh)
+        preh = torch.empty((B, Hd, P), dtype=BF16, device=self.dev) if keep else None
         pooled = torch.empty((B, Hd), dtype=torch.float32, device=self.dev)
-        nat.row_mean(Hh.data_ptr(), pooled.data_ptr(), B * Hd, P, 1.0 / P, self._stream())
+        if C in (32, 64) and Hd in (32, 64) and P >= 64 and P % 8 == 0:
+            # the head's activations are only averaged: sums per tile of 128 pixels instead
+            # of storing and reading them (FIG)
+            part = torch.empty((B, -(-P // 128), Hd), dtype=torch.float32, device=self.dev)
+            nat.mix_mean(p["Q1"].h.data_ptr(), V.data_ptr(), p["q1"].w.data_ptr(), _p(preh), part.data_ptr(),
+                         pooled.data_ptr(), B, Hd, C, P, 1.0 / P, self._stream())
+        else:
+            Hh = torch.empty((B, Hd, P), dtype=BF16, device=self.dev)
+            self._gemm(Hd, P, C, p["Q1"].h, C, V, P, batch=B, sb=C * P, outh=Hh, sc=Hd * P, bias_m=p["q1"].w, act=1,
+                       pre=preh)
+            nat.row_mean(Hh.data_ptr(), pooled.data_ptr(), B * Hd, P, 1.0 / P, self._stream())
         pooled_h = pooled.to(BF16)
         out = torch.empty((B, self.n_out), dtype=torch.float32, device=self.dev)
         self._gemm(B, self.n_out, Hd, pooled_h, Hd, p["Q2"].h, Hd, tb=1, outf=out, bias_n=p["q2"].w)

@@ -478,6 +478,12 @@ int bz_spectral_mix_bwd(const void* dO, const void* U, const void* W, void* dU, 
 int bz_gelu_bwd(const void* dy, const void* pre, void* dx, int64_t n, void* stream);
 /* out[r] = scale * sum_p x[r][p] (bf16 rows of length P, f32 out). */
 int bz_row_mean(const void* x, float* out, int64_t rows, int32_t P, float scale, void* stream);
+/* mean[b][m] = scale * sum_p GELU(W X[b] + bias)[m][p], W [M][K], X [b][K][P] bf16; the
+ * activations are rounded to bf16 as bz_gemm_bf16 would store them, but not stored; pre (or
+ * NULL) takes the bf16 pre-activations [b][M][P]. M, K: 32 or 64. P: a multiple of 8, >= 64;
+ * X on 16 bytes. part: batch * ceil(P / 128) * M floats of scratch. */
+int bz_mix_mean(const void* W, const void* X, const float* bias, void* pre, float* part, float* mean,
+                int32_t batch, int32_t M, int32_t K, int32_t P, float scale, void* stream);
 /* x[r][p] = scale * g[r] (bf16 out). */
 int bz_row_broadcast(const float* g, void* x, int64_t rows, int32_t P, float scale, void* stream);
 /* out[c] += sum_b sum_p x[b][c][p] (bf16 [B][C][P], f32 out). */

@@ -436,6 +436,40 @@ def test_lift_layer_matches_general_kernel(bz, K, N, batch):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("keep", [False, True])
+@pytest.mark.parametrize("M,K,P,batch", [(32, 32, 64, 1), (64, 32, 128, 2), (32, 64, 136, 3), (64, 64, 1000, 5),
+                                         (64, 32, 14400, 9)])
+def test_fused_head_mean_matches_stored_activations(bz, M, K, P, batch, keep):
+    """The mixing kernel's channel means against its stored activations averaged in float64:
+    only the order of the f32 additions differs (at most P, each within 2^-24 of the sum of
+    magnitudes; P / 32 + 16 covers the tree and the tiles). Pre-activations bit for bit."""
+    from beamz_b200 import _native as nat
+
+    g = torch.Generator().manual_seed(M * K + P)
+    W = (torch.randn(M, K, generator=g) / K ** 0.5).to(torch.bfloat16).cuda()
+    X = torch.randn(batch, K, P, generator=g).to(torch.bfloat16).cuda()
+    bias = torch.randn(M, generator=g).cuda()
+    st = torch.cuda.current_stream().cuda_stream
+    H = torch.empty(batch, M, P, dtype=torch.bfloat16, device="cuda")
+    pres = [torch.empty_like(H) if keep else None for _ in range(2)]
+    q = nat.Gemm()
+    q.M, q.N, q.K, q.batch, q.splitk, q.act, q.alpha = M, P, K, batch, 1, 1, 1.0
+    q.A, q.lda, q.B, q.ldb, q.sb = W.data_ptr(), K, X.data_ptr(), P, K * P
+    q.bias_m, q.outh, q.ldc, q.sc = bias.data_ptr(), H.data_ptr(), P, M * P
+    if keep:
+        q.pre, q.ldpre, q.spre = pres[0].data_ptr(), P, M * P
+    nat.gemm(q, st)
+    part = torch.empty(batch, -(-P // 128), M, device="cuda")
+    mean = torch.empty(batch, M, device="cuda")
+    nat.mix_mean(W.data_ptr(), X.data_ptr(), bias.data_ptr(), pres[1].data_ptr() if keep else None, part.data_ptr(),
+                 mean.data_ptr(), batch, M, K, P, 1.0 / P, st)
+    want = H.double().mean(2)
+    bound = (P / 32 + 16) * 2.0 ** -24 * H.double().abs().mean(2) + 1e-12
+    assert bool(((mean.double() - want).abs() <= bound).all())
+    if keep:
+        assert torch.equal(pres[0], pres[1])
+
+
 def test_fno_with_tcgen05_spectral_gemms_matches_oracle(bz):
     """n = 64, 8 modes, width 32, batch 8: the DFT GEMMs (M = 256, N = 256, K = 4096)
     and their inverses run on the tcgen05 kernel."""
