@@ -335,6 +335,40 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity, int limi
   return false;
 }
 
+// tcgen05.ld, tcgen05.dealloc and the aligned cluster barrier are executed by a whole warp
+// together. A warp may come from code that its lanes took on different paths (rows or pixels
+// past the end store nothing), and nothing but __syncwarp() promises that it is whole again.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+template <int PAIR>  // CTAs the columns were allocated for
+__device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t columns) {
+  __syncwarp();
+  if constexpr (PAIR == 2)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(columns));
+  else
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(columns));
+}
+
 __global__ void __launch_bounds__(tc::THREADS) gemm_tc_kernel(GemmP p) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -449,11 +483,7 @@ __global__ void __launch_bounds__(tc::THREADS) gemm_tc_kernel(GemmP p) {
     for (int c0 = 0; c0 < tc::BN; c0 += 8) {
       uint32_t v[8];
       if (kt0 < kt1) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-            : "r"(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        tmem_ld8(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
       } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = 0u;
@@ -479,7 +509,7 @@ __global__ void __launch_bounds__(tc::THREADS) gemm_tc_kernel(GemmP p) {
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(tc::BN));
+  if (warp == 0) tmem_free<1>(taddr, tc::BN);
 }
 
 int launch_gemm_tc(const GemmP& p, cudaStream_t st) {
@@ -629,11 +659,7 @@ __global__ void __launch_bounds__(tc::THREADS) gemm_tma_kernel(const __grid_cons
     for (int c0 = 0; c0 < tc::BN; c0 += 8) {
       uint32_t v[8];
       if (nt > 0) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-            : "r"(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        tmem_ld8(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
       } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = 0u;
@@ -674,7 +700,7 @@ __global__ void __launch_bounds__(tc::THREADS) gemm_tma_kernel(const __grid_cons
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(tc::BN));
+  if (warp == 0) tmem_free<1>(taddr, tc::BN);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -724,18 +750,6 @@ int launch_gemm_tma(const GemmP& p, cudaStream_t st) {
   gemm_tma_kernel<<<grid, tc::THREADS, tma::SMEM, st>>>(ma, mb, p);
   const int rc = check_launch("bz_gemm_bf16");
   return rc == BZ_OK ? 1 : rc;
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
 // ---- tcgen05 + TMA path on CTA pairs: 256 x 256 tiles, persistent -----------------------
@@ -801,6 +815,7 @@ __device__ __forceinline__ void commit_pair(uint32_t mbar) {  // the barrier at 
 }
 
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
@@ -914,7 +929,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
     int n_acc = 0;
     for (int t = first; t < total; t += stride, ++n_acc) {
       const int acc = n_acc & 1;
-      if (!tc_wait(tfull0 + 8 * acc, (uint32_t)((n_acc / 2) & 1))) {
+      // one outcome for the warp: its lanes poll on their own, and may give up apart
+      if (!__all_sync(0xffffffffu, tc_wait(tfull0 + 8 * acc, (uint32_t)((n_acc / 2) & 1)))) {
         ok = false;
         break;
       }
@@ -983,8 +999,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
   if (!__syncthreads_and(ok) && threadIdx.x == 0) atomicExch(&g_tc_error, 1);
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   cluster_sync();  // neither CTA leaves while the other may still signal it
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(2 * pair::BN));
+  if (warp == 0) tmem_free<2>(taddr, 2 * pair::BN);
   cluster_sync();
 }
 
@@ -1288,8 +1303,7 @@ __global__ void __launch_bounds__(mix::THREADS) mix_tc_kernel(const __grid_const
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(2 * C::NCOL));
+  if (warp == 0) tmem_free<1>(taddr, 2 * C::NCOL);
 }
 
 // The mixing kernel takes: one weight for the whole batch (sa == 0), X (B operand,
@@ -1406,6 +1420,7 @@ __global__ void __launch_bounds__(256) lift_kernel(GemmP p, int groups) {
       return k < p.K && n0 + pix < p.N ? __ldg(X + (long long)k * p.ldb + pix) : (unsigned short)0;
     };
     const unsigned b0 = pack(x(2 * q), x(2 * q + 1)), b1 = pack(x(2 * q + 8), x(2 * q + 9));
+    __syncwarp();  // the lanes' loads differ (padding, the last pixels); mma.sync takes the whole warp
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
 #pragma unroll
@@ -1563,7 +1578,7 @@ __global__ void __launch_bounds__(wg::THREADS) wgrad_tc_kernel(const __grid_cons
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(NCOL));
+  if (warp == 0) tmem_free<1>(taddr, NCOL);
 }
 
 // The weight-gradient kernel takes: ta = 0, tb = 1, atomic with sc = 0 (a sum over the
