@@ -324,20 +324,21 @@ class Engine3D:
         self.d2h_bytes += out.nbytes
         return out
 
-    def collect_monitors(self, recs, times):
-        """Fill plane monitors from the device records (monitors.py:317-396, 426-439)."""
+    def collect_monitors(self, recs, times, steps):
+        """Fill plane monitors from the device records (monitors.py:317-396, 426-439):
+        row i was recorded at step steps[i], time times[i]."""
         if recs is not None:
             for m, sl, shp in zip(self.mons, self.mon_slices, self.mon_shape):
                 part = recs[:, 0, :, sl, :]  # [steps][comp][points][6]
                 vals = part[:, 0] + 1j * part[:, 1] if self.n_comp == 2 else part[:, 0]
                 k = m.record_interval
-                sel = np.arange(k - 1, len(times), k) if k > 1 else np.arange(len(times))
+                sel = np.flatnonzero((steps + 1) % k == 0) if k > 1 else np.arange(len(steps))
                 for n in sel:
                     comps = [vals[n, :, q].reshape(shp) for q in range(6)]
                     if self.n_comp == 2:
                         comps = [c.astype(np.complex128) for c in comps]
                     m._append_3d(comps, times[n])
-                    m.last_record_step = int(n)
+                    m.last_record_step = int(steps[n])
                 m._manage_memory()
         if self.dft is not None:
             self._fold()

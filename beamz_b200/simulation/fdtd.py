@@ -258,12 +258,17 @@ class FDTD:
         eng = self.engine
         on_device = eng.take_records_device() if hasattr(eng, "take_records_device") else None
         recs = eng.take_records() if on_device is None and hasattr(eng, "take_records") else None
-        steps = np.arange(eng.step_index)
-        times = np.zeros(len(steps))
-        if len(steps) > 1:
-            times[1:] = np.cumsum(np.full(len(steps) - 1, self.dt))
+        rows = on_device if on_device is not None else recs
+        # the rows end with the step just taken; those of steps before the first one here
+        # went to the monitors when the run was finalised earlier
+        first = eng.step_index - (0 if rows is None else len(rows))
+        steps = np.arange(first, eng.step_index)
+        times = np.zeros(eng.step_index)
+        if len(times) > 1:
+            times[1:] = np.cumsum(np.full(len(times) - 1, self.dt))
+        times = times[first:]
         if hasattr(eng, "collect_monitors"):
-            eng.collect_monitors(recs, times)
+            eng.collect_monitors(recs, times, steps)
             return
         if on_device is not None:
             self._load_device_records(eng, on_device, times, steps)
@@ -276,8 +281,8 @@ class FDTD:
         widened to float64 on the device and arrive in page-locked memory at copy speed (a
         four-line record of 2000 steps: 45 ms of host conversions before)."""
         for mon, sl in zip(eng.mp.monitors, eng.mp.slices):
-            k = mon.record_interval
-            sel = slice(k - 1, None, k) if k > 1 else slice(None)
+            k = mon.record_interval  # rows of the steps k - 1, 2 k - 1, ...
+            sel = slice((k - 1 - int(steps[0])) % k, None, k) if k > 1 else slice(None)
             part = recs[sel, 0, :, sl, :].double()  # [steps][comp][points][3]
             vals = torch.complex(part[:, 0], part[:, 1]) if eng.n_comp == 2 else part[:, 0]
             ez, hx, hy = vals.unbind(-1)
@@ -302,14 +307,13 @@ class FDTD:
             part = recs[:, 0, :, sl, :]  # [steps][comp][points][3]
             vals = part[:, 0] + 1j * part[:, 1] if eng.n_comp == 2 else part[:, 0]
             k = mon.record_interval
-            sel = np.arange(k - 1, len(steps), k) if k > 1 else np.arange(len(steps))
-            sel = sel[sel >= 0]
+            sel = np.flatnonzero((steps + 1) % k == 0) if k > 1 else np.arange(len(steps))
             vals = vals[sel]
             ez, hx, hy = vals[..., 0], vals[..., 1], vals[..., 2]
             if eng.n_comp == 2:
                 ez, hx, hy = ez.astype(np.complex128), hx.astype(np.complex128), hy.astype(np.complex128)
             mon.load_record_2d(ez, hx, hy, times[sel])
-            mon.last_record_step = int(sel[-1]) if len(sel) else mon.last_record_step
+            mon.last_record_step = int(steps[sel[-1]]) if len(sel) else mon.last_record_step
 
     def _collect_dft(self):
         eng = self.engine

@@ -65,3 +65,45 @@ def test_mode_overlap_matches_oracle(bz, precision, tol):
     assert got.shape == want.shape == (3,)
     assert np.all(want > 0.05)
     np.testing.assert_allclose(got, want, rtol=tol)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("interval", [1, 3])
+def test_finalise_continue_finalise_equals_one_run(bz, dims, interval):
+    """run_for / finalize_simulation / run_for / finalize_simulation: the monitor's samples,
+    times and power equal those of the run finalised once."""
+    got = []
+    for parts in ((100,), (40, 60), (37, 1, 62)):
+        if dims == 2:
+            d = D.wg_design(bz)
+            t = D.time_axis(bz, 100)
+            d += bz.GaussianSource(position=(1.0 * D.UM, 1.0 * D.UM), width=0.1 * D.UM, signal=D.gauss_signal(bz, t))
+            mon = bz.Monitor(design=d, start=(1.6 * D.UM, 0.6 * D.UM), end=(1.6 * D.UM, 1.4 * D.UM),
+                             record_interval=interval)
+            grid = bz.RegularGrid
+            res = D.RES
+        else:
+            res = 30e-9
+            d = bz.Design(width=20.5 * res, height=16.5 * res, depth=12.5 * res, material=bz.Material(2.0), pml_size=3 * res)
+            t = np.arange(100) * 0.99 * res / (bz.LIGHT_SPEED * np.sqrt(3))
+            d += bz.GaussianSource(position=(8 * res, 8 * res, 6 * res), width=res / 10, signal=np.sin(2e15 * t))
+            mon = bz.Monitor(design=d, start=(0.0, 4 * res, 4 * res), plane_normal="x", plane_position=12 * res,
+                             size=(8 * res, 4 * res), record_interval=interval)
+            grid = lambda d_, r_: bz.RegularGrid3D(d_, r_, extrude=True)  # noqa: E731
+        d += mon
+        sim = bz.FDTD(design=grid(d, res), time=t, backend_options={"precision": "fp64"})
+        for n in parts:
+            sim.run_for(n, live=False, save=False, save_memory_mode=True)
+            sim.finalize_simulation()
+        got.append(mon)
+    one = got[0]
+    assert len(one.fields["t"]) == 100 // interval and np.abs(np.array(one.fields["Ez"])).max() > 0
+    for mon in got[1:]:
+        assert set(mon.fields) == set(one.fields)
+        for k, v in one.fields.items():
+            np.testing.assert_array_equal(np.array(mon.fields[k]), np.array(v), err_msg=k)
+        np.testing.assert_array_equal(mon.power_timestamps, one.power_timestamps)
+        np.testing.assert_allclose(mon.power_history, one.power_history, rtol=1e-13)
+        np.testing.assert_allclose(mon.power_accumulated, one.power_accumulated, rtol=1e-13)
+        assert mon.power_accumulation_count == one.power_accumulation_count
+        assert mon.last_record_step == one.last_record_step
