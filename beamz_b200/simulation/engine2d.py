@@ -308,12 +308,15 @@ class Engine2D:
 
         Every candidate gives the same results (same arithmetic per cell), and a launch
         only writes the copy that the next step overwrites and ring/record slots of steps
-        not yet taken, so timing from the current state changes nothing. Each candidate
+        not yet taken, so timing from the current state changes nothing: monitor samples
+        whose ring slots those steps come round to are folded first. Each candidate
         is launched once to warm up, then timed over ``launches`` launches in ``rounds``
         interleaved rounds (best time kept). The choice is cached per (device, grid,
         designs, components, dtype) for the process."""
         key = (torch.cuda.get_device_name(self.dev), self.nx, self.ny, self.n_designs, self.n_comp, self.bz_dtype)
         if key not in _TUNED:
+            if self.step_index - self._folded > RING_LEN - max(tb for tb, _ in candidates):
+                self._fold()
             times = {c: float("inf") for c in candidates}
             for tb, tile in candidates:
                 self.time_block, self.tb_tile = tb, tile

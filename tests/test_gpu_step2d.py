@@ -253,6 +253,28 @@ def test_blocked_power_matches_single_steps(bz, nx, ny, precision):
     assert rel_l2(outs[1][0], outs[0][0]) <= 1e-13
 
 
+@pytest.mark.parametrize("n_before", [3, 55, 56, 60, 63])
+def test_tuning_keeps_samples_waiting_in_the_ring(bz, n_before):
+    """Single steps leave monitor samples in the ring; the first run_steps of a shape then
+    times its launches. The DFT sums equal those of an engine that tunes nothing."""
+    from beamz_b200.simulation import engine2d
+
+    eps, sigma, dx, dt, t, sig, _ = _random_problem(11)
+    src = bz.GaussianSource(position=(18 * dx, 14 * dx), width=dx / 10, signal=sig)
+    mon = bz.Monitor(start=(4 * dx, 14 * dx), end=(30 * dx, 14 * dx), frequencies=[1.9e14, 2.1e14])
+    dfts = []
+    for block in (7, "auto"):
+        engine2d._TUNED.clear()
+        eng = engine2d.Engine2D(eps, sigma, dx, dx, dt, len(t), [src], [mon], precision="fp64", n_comp=1,
+                                record=False, use_graphs=False, time_block=block)
+        for _ in range(n_before):
+            eng.step_once()
+        eng.run_steps(len(t) - n_before)
+        dfts.append(eng.dft_fields())
+    assert engine2d._TUNED and np.abs(dfts[0]).max() > 0
+    assert rel_l2(dfts[1], dfts[0]) <= 1e-12
+
+
 def test_graph_replay_equals_direct_launches(bz):
     eps, sigma, dx, dt, t, sig, _ = _random_problem(5, n_steps=300)
     src = bz.GaussianSource(position=(18 * dx, 14 * dx), width=dx / 10, signal=sig)
