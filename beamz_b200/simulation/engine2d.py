@@ -22,6 +22,15 @@ from .guard import DivergenceGuard
 
 GRAPH_CHUNK = 64  # at most this many steps per captured graph
 POWER_BLOCK = 7  # steps of a blocked launch that accumulates power
+# A CUDA graph saves the host a few us a launch and costs its capture (0.3 ms with blocked
+# launches, 1 ms with one step a launch), so runs shorter than this do without (ms with /
+# without a graph). One step a launch (power of complex fields, time_block 1): 200 x 150
+# complex cells with power, 256 steps 8.5 / 8.2, 512 15.0 / 15.1, 1000 27.3 / 28.1, 4000
+# 102.5 / 108.4; 61 x 47 cells 6.6 / 6.4, 11.2 / 11.1, 20.1 / 21.0, 75.1 / 79.6. Blocks of 5 to 9
+# steps: 61 x 47, 2000 steps 4.13 / 4.18, 3000 5.33 / 5.63, 4000 6.76 / 7.17; 500 x 300 with
+# power 7.17 / 7.11, 9.50 / 9.71, 11.96 / 12.35; 601 x 397 in float64, whose launches take the
+# GPU longer than the host, 7.55 / 7.35, 10.37 / 10.20, 13.09 / 13.08.
+GRAPH_MIN_STEPS_SINGLE, GRAPH_MIN_STEPS_BLOCKED = 512, 3072
 RING_LEN = GRAPH_CHUNK  # monitor samples kept between DFT folds
 # (steps per launch, register-tile shape) tried by the autotuner: the large tile for grids
 # that fill the GPU several times over, smaller ones (less halo work per block, more
@@ -74,7 +83,6 @@ class Engine2D:
         self._setup_sources()
         self._setup_monitors(monitors, record)
         self.d_step = torch.zeros(1, dtype=torch.int64, device=self.dev)
-        self.use_graphs = use_graphs
         self._graphs: dict[int, torch.cuda.CUDAGraph] = {}
         self.kernel_timer = None  # graphs.KernelTimer around the step launches (direct launches only)
         self._autotune = time_block == "auto"
@@ -89,6 +97,9 @@ class Engine2D:
             self.time_block = POWER_BLOCK if n_comp == 1 else 1
         self._autotune = self._autotune and not power
         self.tb_tile = int(tb_tile)
+        if use_graphs == "auto":  # tuning never picks single steps
+            use_graphs = self.n_steps >= (GRAPH_MIN_STEPS_SINGLE if self.time_block == 1 else GRAPH_MIN_STEPS_BLOCKED)
+        self.use_graphs = use_graphs
         # steps per graph: an even number of steps keeps the copy parity, so one
         # graph serves every chunk of a run
         self.chunk = GRAPH_CHUNK // (2 * self.time_block) * (2 * self.time_block)

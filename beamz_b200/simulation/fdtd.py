@@ -28,12 +28,6 @@ from .meshing import BaseMeshGrid, RegularGrid, RegularGrid3D, to_host
 
 __all__ = ["FDTD"]
 
-# CUDA graphs pay where the host cannot issue launches as fast as they run. A blocked 2D
-# launch of 5-9 steps takes the GPU 11 us at the least and the host about as long, so only
-# long runs gain their capture back (with / without: 150 steps of 61 x 47 cells 1.89 / 1.53
-# ms, 1000 of 601 x 397 in float64 5.6 / 5.3, 2000 of 1000 x 500 complex 11.3 / 11.2). A 3D
-# step is three launches of a few us on a small grid and needs them.
-GRAPH_MIN_STEPS_2D = 4096
 PINNED_RECORD_BYTES = 128 << 20  # a monitor's samples above this go to pageable memory
 
 
@@ -115,9 +109,9 @@ class FDTD:
         opts = self.backend_options
         precision = opts.get("precision", "fp32")
         n_comp = opts.get("n_comp")
-        graphs = opts.get("graph")
-        if graphs is None:
-            graphs = self.is_3d or self.num_steps >= GRAPH_MIN_STEPS_2D
+        # not given: a 3D step is three launches of a few us on a small grid and needs graphs,
+        # a 2D engine decides by the length of its launches
+        graphs = opts.get("graph", True if self.is_3d else "auto")
         if self.is_3d:
             from .engine3d import Engine3D
 

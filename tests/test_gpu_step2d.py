@@ -275,6 +275,19 @@ def test_tuning_keeps_samples_waiting_in_the_ring(bz, n_before):
     assert rel_l2(dfts[1], dfts[0]) <= 1e-12
 
 
+@pytest.mark.parametrize("steps,cplx,opts,want", [
+    (511, True, {}, False), (512, True, {}, True), (1000, False, {"time_block": 1}, True), (511, False, {"time_block": 1}, False),
+    (1000, False, {}, False), (3072, False, {}, True), (1000, False, {"graph": True}, True), (3072, True, {"graph": False}, False)])
+def test_graphs_by_default_follow_the_launch_length(bz, steps, cplx, opts, want):
+    """Runs of one step a launch (power of complex fields, time_block 1) replay graphs from
+    512 steps on, blocked ones from 3072; the option overrides either."""
+    eps, sigma, dx, dt, t, sig, _ = _random_problem(2, n_steps=steps)
+    src = bz.GaussianSource(position=(18 * dx, 14 * dx), width=dx / 10, signal=sig)
+    sim = _sim_from_arrays(bz, eps, sigma, dx, t, [src], [], "fp32", n_comp=2 if cplx else 1, **opts)
+    sim.run(live=False, save=False, save_memory_mode=True, accumulate_power=cplx)
+    assert sim.engine.step_index == steps and bool(sim.engine._graphs) == want
+
+
 def test_graph_replay_equals_direct_launches(bz):
     eps, sigma, dx, dt, t, sig, _ = _random_problem(5, n_steps=300)
     src = bz.GaussianSource(position=(18 * dx, 14 * dx), width=dx / 10, signal=sig)
