@@ -184,6 +184,7 @@ class FNO2d:
             part = torch.empty((B, -(-P // 128), Hd), dtype=torch.float32, device=self.dev)
             nat.mix_mean(p["Q1"].h.data_ptr(), V.data_ptr(), p["q1"].w.data_ptr(), _p(preh), part.data_ptr(),
                          pooled.data_ptr(), B, Hd, C, P, 1.0 / P, self._stream())
+            self.flops += 2.0 * Hd * P * C * B
         else:
             Hh = torch.empty((B, Hd, P), dtype=BF16, device=self.dev)
             self._gemm(Hd, P, C, p["Q1"].h, C, V, P, batch=B, sb=C * P, outh=Hh, sc=Hd * P, bias_m=p["q1"].w, act=1,

@@ -470,6 +470,20 @@ def test_fused_head_mean_matches_stored_activations(bz, M, K, P, batch, keep):
         assert torch.equal(pres[0], pres[1])
 
 
+@pytest.mark.parametrize("n,width,head", [(64, 32, 64), (64, 32, 48), (30, 32, 64)])
+def test_flops_count_every_product_of_a_prediction(bz, n, width, head):
+    """FNO2d.flops after one prediction: lift, transforms, 1x1 layers and both head layers,
+    whether the head's means are taken inside the mixing kernel or not."""
+    from beamz_b200.surrogate.fno import FNO2d
+
+    B, modes, layers = 2, 4, 2
+    net = FNO2d(n=n, width=width, modes=modes, layers=layers, head=head, n_out=3)
+    net.forward(torch.rand(B, n, n))
+    P, K2 = n * n, 4 * modes * modes
+    layer = 2 * 2 * width * P * K2 + 2 * width * width * P
+    assert net.flops == B * (2 * width * P * 3 + layers * layer + 2 * head * width * P + 2 * head * 3)
+
+
 def test_fno_with_tcgen05_spectral_gemms_matches_oracle(bz):
     """n = 64, 8 modes, width 32, batch 8: the DFT GEMMs (M = 256, N = 256, K = 4096)
     and their inverses run on the tcgen05 kernel."""
