@@ -152,6 +152,7 @@ _adam = _sig("bz_adam", C.c_int, [vp, vp, vp, vp, vp, i64, C.c_float, C.c_float,
 _to_bf16 = _sig("bz_to_bf16", C.c_int, [vp, vp, i64, vp])
 _gemm_err = _sig("bz_gemm_error", C.c_int, [C.POINTER(i32), i32])
 _gemm_selftest = _sig("bz_gemm_wait_selftest", C.c_int, [vp, vp, vp, i32, vp])
+_gemm_pair_selftest = _sig("bz_gemm_pair_wait_selftest", C.c_int, [vp, vp, vp, i32, i32, vp])
 _field_check = _sig("bz_field_check", C.c_int, [vp, i32, i64, f64, i64, vp, vp])
 
 #: every symbol include/beamz_b200.h declares (checked by the CPU test suite)
@@ -159,7 +160,7 @@ EXPORTED = ["bz_version", "bz_last_error", "bz_step2d", "bz_step2d_multi", "bz_s
             "bz_adjoint_step2d", "bz_adjoint_step2d_multi", "bz_step3d", "bz_cell_ops", "bz_gather", "bz_power3d", "bz_dft_fold_q", "bz_rasterize3d", "bz_prepare_coeffs", "bz_update_h2d",
             "bz_update_e2d", "bz_rasterize2d", "bz_gemm_bf16", "bz_spectral_mix", "bz_spectral_mix_bwd", "bz_gelu_bwd",
             "bz_row_mean", "bz_mix_mean", "bz_row_broadcast", "bz_chan_sum", "bz_adam", "bz_to_bf16", "bz_gemm_error",
-            "bz_gemm_wait_selftest", "bz_field_check"]
+            "bz_gemm_wait_selftest", "bz_gemm_pair_wait_selftest", "bz_field_check"]
 
 
 class NativeError(RuntimeError):
@@ -313,6 +314,11 @@ def field_check(ptr: int, dtype: int, n: int, limit: float, step: int, status_pt
 def gemm_wait_selftest(a_ptr: int, b_ptr: int, c_ptr: int, wait_limit: int, stream) -> int:
     """Status of the tcgen05 GEMM's withheld-slice run (BZ_ERR_TIMEOUT expected); does not raise."""
     return _gemm_selftest(vp(a_ptr), vp(b_ptr), vp(c_ptr), int(wait_limit), vp(stream))
+
+
+def gemm_pair_wait_selftest(a_ptr: int, b_ptr: int, c_ptr: int, wait_limit: int, withhold: int, stream) -> int:
+    """As gemm_wait_selftest, of the CTA-pair kernel (A and C of 256 rows)."""
+    return _gemm_pair_selftest(vp(a_ptr), vp(b_ptr), vp(c_ptr), int(wait_limit), int(withhold), vp(stream))
 
 
 def gemm_error(reset: bool = True) -> int:

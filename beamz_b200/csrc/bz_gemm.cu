@@ -49,8 +49,8 @@ struct GemmP {
   bf16* pre;
   long long ldpre, spre;
   const bf16* cadd_h;  // the added term in bf16 instead of f32 (same strides), or null
-  int wait_limit;  // polls of a bounded mbarrier wait before it gives up (tcgen05 kernel)
-  int withhold;    // 1: the tcgen05 kernel issues no MMA for its first K slice (timeout self-test)
+  int wait_limit;  // polls of a bounded mbarrier wait before it gives up (tcgen05 kernels)
+  int withhold;    // 1: no MMA for the first K slice, in the pair kernel for any (timeout self-tests)
 };
 
 __device__ __forceinline__ float gelu_f(float v) {
@@ -763,7 +763,8 @@ int launch_gemm_tma(const GemmP& p, cudaStream_t st) {
 // 32 KB stages; both CTAs' copies complete on the even CTA's barrier), warp 1 of the even
 // CTA issues the MMAs, warps 2-5 run the epilogue. tcgen05.commit frees a stage in both
 // CTAs at once. Every output element sums its K slices in the same
-// order as in the single-CTA kernel: the same bits. Waits are bounded as above.
+// order as in the single-CTA kernel: the same bits. Waits are bounded as above; those that
+// only see issued copies and MMAs end, at the end, by the longer compiled-in limit.
 // M x N x K, us, single-CTA kernel -> this one: 2048 x 1024 x 14400 in two K splits 93 ->
 // 52; 2048 x 14400 x 1024 92 -> 56; 8192 x 1024 x 14400 275 -> 179 (1350 TFLOP/s); 8192 x
 // 14400 x 1024 307 -> 194. Passing the odd CTA's landed stages on with a remote arrive
@@ -777,8 +778,8 @@ constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >
 }  // namespace pair
 
 // Bounded wait whose success orders what a thread of the other CTA did before its arrive.
-__device__ __forceinline__ bool tc_wait_cluster(uint32_t mbar, uint32_t parity) {
-  for (int i = 0; i < tc::WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool tc_wait_cluster(uint32_t mbar, uint32_t parity, int limit) {
+  for (int i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -861,6 +862,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
     k0 = ks * kper;
     k1 = min(ktiles, k0 + kper);
   };
+  const int limit = p.wait_limit;
   bool ok = true;
   if (warp == 0 && lane == 0) {  // ---- loads: both CTAs' copies complete on the even CTA's barrier
     uint32_t full_r0;
@@ -873,7 +875,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
       k_range(t, k0, k1);
       for (int k = k0; k < k1; ++k, ++it) {
         const int s = it % pair::S;
-        if (it >= pair::S && !tc_wait(empty0 + 8 * s, (uint32_t)((it / pair::S - 1) & 1))) {
+        if (it >= pair::S && !tc_wait(empty0 + 8 * s, (uint32_t)((it / pair::S - 1) & 1), limit)) {
           ok = false;
           break;
         }
@@ -890,18 +892,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
         if (!tc_wait(full0 + 8 * (j % pair::S), (uint32_t)((j / pair::S) & 1))) ok = false;
   } else if (warp == 1 && lane == 0 && rank == 0) {
     int it = 0, n_acc = 0;
-    for (int t = first; t < total && ok; t += stride, ++n_acc) {
+    for (int t = p.withhold ? total : first; t < total && ok; t += stride, ++n_acc) {
       int k0, k1;
       k_range(t, k0, k1);
       const int acc = n_acc & 1;
-      if (n_acc >= 2 && !tc_wait_cluster(tempty0 + 8 * acc, (uint32_t)((n_acc / 2 - 1) & 1))) {
+      if (n_acc >= 2 && !tc_wait_cluster(tempty0 + 8 * acc, (uint32_t)((n_acc / 2 - 1) & 1), limit)) {
         ok = false;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
       for (int k = k0; k < k1; ++k, ++it) {
         const int s = it % pair::S;
-        if (!tc_wait(full0 + 8 * s, (uint32_t)((it / pair::S) & 1))) {
+        if (!tc_wait(full0 + 8 * s, (uint32_t)((it / pair::S) & 1), limit)) {
           ok = false;
           break;
         }
@@ -920,17 +922,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
       }
       if (ok) commit_pair(tfull0 + 8 * acc);
     }
-    if (!ok) {  // let issued MMAs drain before the TMEM goes
-      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done));
-      tc_wait(done, 0u);
-    }
+    // issued MMAs have ended before the TMEM goes, also where the epilogue gave up on them
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(done));
+    if (!tc_wait(done, 0u)) ok = false;
   } else if (warp >= 2) {  // ---- epilogue: warp w owns accumulator rows 32 (w % 4) ...
     const int quad = warp & 3;
     int n_acc = 0;
     for (int t = first; t < total; t += stride, ++n_acc) {
       const int acc = n_acc & 1;
       // one outcome for the warp: its lanes poll on their own, and may give up apart
-      if (!__all_sync(0xffffffffu, tc_wait(tfull0 + 8 * acc, (uint32_t)((n_acc / 2) & 1)))) {
+      if (!__all_sync(0xffffffffu, tc_wait(tfull0 + 8 * acc, (uint32_t)((n_acc / 2) & 1), limit))) {
         ok = false;
         break;
       }
@@ -1989,32 +1990,49 @@ extern "C" int bz_mix_mean(const void* W, const void* X, const float* bias, void
   return bz::check_launch("bz_mix_mean");
 }
 
-extern "C" int bz_gemm_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, void* stream) {
-  BZ_REQUIRE(A && B && C, "bz_gemm_wait_selftest: NULL buffer");
-  BZ_REQUIRE(wait_limit >= 1, "bz_gemm_wait_selftest: wait_limit must be positive");
+// Runs one tile of M x 256 x 64 that cannot complete and reads the error word.
+static int wait_selftest(const char* name, int M, const void* A, const void* B, float* C, int32_t wait_limit,
+                         int32_t withhold, void* stream) {
+  BZ_REQUIRE(A && B && C, "%s: NULL buffer", name);
+  BZ_REQUIRE(wait_limit >= 1, "%s: wait_limit must be positive", name);
   bz::GemmP p = {};
-  p.M = 128; p.N = 256; p.K = 64; p.batch = 1; p.splitk = 1;
+  p.M = M; p.N = 256; p.K = 64; p.batch = 1; p.splitk = 1;
   p.A = (const bz::bf16*)A; p.lda = 64;
   p.B = (const bz::bf16*)B; p.ldb = 64;
   p.alpha = 1.0f;
   p.outf = C; p.ldc = 256;
   p.wait_limit = wait_limit;
-  p.withhold = 1;
+  p.withhold = withhold;
   cudaStream_t st = bz::as_stream(stream);
   const int zero = 0;
   if (cudaMemcpyToSymbolAsync(bz::g_tc_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return bz::fail(BZ_ERR_CUDA, "bz_gemm_wait_selftest: cannot reset the error word");
-  const int rc = bz::launch_gemm_tc(p, st);
-  if (rc != BZ_OK) return rc;
-  if (cudaStreamSynchronize(st) != cudaSuccess) return bz::fail(BZ_ERR_CUDA, "bz_gemm_wait_selftest: launch failed");
+    return bz::fail(BZ_ERR_CUDA, "%s: cannot reset the error word", name);
+  if (M == bz::pair::BM) {
+    const int t = bz::launch_gemm_pair(p, st);
+    if (t < 0) return t;
+    if (t == 0) return bz::fail(BZ_ERR_UNSUPPORTED, "%s: the pair kernel does not run here", name);
+  } else {
+    const int rc = bz::launch_gemm_tc(p, st);
+    if (rc != BZ_OK) return rc;
+  }
+  if (cudaStreamSynchronize(st) != cudaSuccess) return bz::fail(BZ_ERR_CUDA, "%s: launch failed", name);
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, bz::g_tc_error, sizeof(int)) != cudaSuccess)
-    return bz::fail(BZ_ERR_CUDA, "bz_gemm_wait_selftest: cannot read the error word");
+    return bz::fail(BZ_ERR_CUDA, "%s: cannot read the error word", name);
   if (cudaMemcpyToSymbol(bz::g_tc_error, &zero, sizeof(int)) != cudaSuccess)
-    return bz::fail(BZ_ERR_CUDA, "bz_gemm_wait_selftest: cannot reset the error word");
-  if (v) return bz::fail(BZ_ERR_TIMEOUT, "bz_gemm_wait_selftest: the withheld slice's wait ran out after %d polls",
-                         wait_limit);
+    return bz::fail(BZ_ERR_CUDA, "%s: cannot reset the error word", name);
+  if (v) return bz::fail(BZ_ERR_TIMEOUT, "%s: the withheld slice's wait ran out after %d polls", name, wait_limit);
   return BZ_OK;
+}
+
+extern "C" int bz_gemm_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, void* stream) {
+  return wait_selftest("bz_gemm_wait_selftest", bz::tc::BM, A, B, C, wait_limit, 1, stream);
+}
+
+extern "C" int bz_gemm_pair_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, int32_t withhold,
+                                          void* stream) {
+  BZ_REQUIRE(withhold == 1, "bz_gemm_pair_wait_selftest: withhold %d", withhold);
+  return wait_selftest("bz_gemm_pair_wait_selftest", bz::pair::BM, A, B, C, wait_limit, withhold, stream);
 }
 
 extern "C" int bz_gemm_error(int32_t* value, int32_t reset) {
