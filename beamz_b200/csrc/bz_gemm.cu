@@ -50,7 +50,8 @@ struct GemmP {
   long long ldpre, spre;
   const bf16* cadd_h;  // the added term in bf16 instead of f32 (same strides), or null
   int wait_limit;  // polls of a bounded mbarrier wait before it gives up (tcgen05 kernels)
-  int withhold;    // 1: no MMA for the first K slice, in the pair kernel for any (timeout self-tests)
+  int withhold;    // timeout self-tests. 1: no MMA for the first K slice, in the pair kernel for any;
+                   // 2, 3: the pair's even, odd CTA does not load the last K slice of a tile
 };
 
 __device__ __forceinline__ float gelu_f(float v) {
@@ -763,8 +764,11 @@ int launch_gemm_tma(const GemmP& p, cudaStream_t st) {
 // 32 KB stages; both CTAs' copies complete on the even CTA's barrier), warp 1 of the even
 // CTA issues the MMAs, warps 2-5 run the epilogue. tcgen05.commit frees a stage in both
 // CTAs at once. Every output element sums its K slices in the same
-// order as in the single-CTA kernel: the same bits. Waits are bounded as above; those that
-// only see issued copies and MMAs end, at the end, by the longer compiled-in limit.
+// order as in the single-CTA kernel: the same bits. Waits are bounded as above. After a wait
+// that ran out the two loading threads may have stopped at different slices: an incomplete
+// tile makes the epilogues of both CTAs give up, and each then leaves its copies in flight
+// the time to land (their bytes count on the even CTA's barriers only, so the odd one cannot
+// see them; handing its slice count over cost the loading loop 1.7 of 51.2 us, first shape below).
 // M x N x K, us, single-CTA kernel -> this one: 2048 x 1024 x 14400 in two K splits 93 ->
 // 52; 2048 x 14400 x 1024 92 -> 56; 8192 x 1024 x 14400 275 -> 179 (1350 TFLOP/s); 8192 x
 // 14400 x 1024 307 -> 194. Passing the odd CTA's landed stages on with a remote arrive
@@ -774,6 +778,7 @@ constexpr int S = 6, BM = 256, BN = 256, BK = 64, THREADS = 192;
 constexpr int A_ST = 128 * BK * 2, STAGE = 2 * A_ST;
 constexpr int NBAR = 2 * S + 5;  // full, empty per stage; tfull[2], tempty[2], done
 constexpr int SMEM = S * STAGE + 1024 + 8 * NBAR + 16;
+constexpr int DRAIN_LIMIT = 1 << 18;  // polls, 22 ms: copies land within microseconds
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }  // namespace pair
 
@@ -873,6 +878,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
       const int n0 = (mn % n_tiles) * pair::BN + (int)rank * 128;
       int k0, k1;
       k_range(t, k0, k1);
+      k1 -= p.withhold == 2 + (int)rank;
       for (int k = k0; k < k1; ++k, ++it) {
         const int s = it % pair::S;
         if (it >= pair::S && !tc_wait(empty0 + 8 * s, (uint32_t)((it / pair::S - 1) & 1), limit)) {
@@ -889,10 +895,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
     }
     if (rank == 0)
       for (int j = max(0, it - pair::S); j < it; ++j)  // all copies of both CTAs have landed before they end
-        if (!tc_wait(full0 + 8 * (j % pair::S), (uint32_t)((j / pair::S) & 1))) ok = false;
+        if (!tc_wait(full0 + 8 * (j % pair::S), (uint32_t)((j / pair::S) & 1), pair::DRAIN_LIMIT)) ok = false;
   } else if (warp == 1 && lane == 0 && rank == 0) {
     int it = 0, n_acc = 0;
-    for (int t = p.withhold ? total : first; t < total && ok; t += stride, ++n_acc) {
+    for (int t = p.withhold == 1 ? total : first; t < total && ok; t += stride, ++n_acc) {
       int k0, k1;
       k_range(t, k0, k1);
       const int acc = n_acc & 1;
@@ -997,9 +1003,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::THREADS)
     }
   }
   __syncwarp();
-  if (!__syncthreads_and(ok) && threadIdx.x == 0) atomicExch(&g_tc_error, 1);
+  const bool fine = __syncthreads_and(ok);
+  if (!fine && threadIdx.x == 0) atomicExch(&g_tc_error, 1);
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   cluster_sync();  // neither CTA leaves while the other may still signal it
+  if (!fine && rank == 1 && threadIdx.x == 0) tc_wait(done, 0u, pair::DRAIN_LIMIT);  // never signalled here: time passes
   if (warp == 0) tmem_free<2>(taddr, 2 * pair::BN);
   cluster_sync();
 }
@@ -1990,15 +1998,15 @@ extern "C" int bz_mix_mean(const void* W, const void* X, const float* bias, void
   return bz::check_launch("bz_mix_mean");
 }
 
-// Runs one tile of M x 256 x 64 that cannot complete and reads the error word.
-static int wait_selftest(const char* name, int M, const void* A, const void* B, float* C, int32_t wait_limit,
+// Runs one tile of M x 256 x K that cannot complete and reads the error word.
+static int wait_selftest(const char* name, int M, int K, const void* A, const void* B, float* C, int32_t wait_limit,
                          int32_t withhold, void* stream) {
   BZ_REQUIRE(A && B && C, "%s: NULL buffer", name);
   BZ_REQUIRE(wait_limit >= 1, "%s: wait_limit must be positive", name);
   bz::GemmP p = {};
-  p.M = M; p.N = 256; p.K = 64; p.batch = 1; p.splitk = 1;
-  p.A = (const bz::bf16*)A; p.lda = 64;
-  p.B = (const bz::bf16*)B; p.ldb = 64;
+  p.M = M; p.N = 256; p.K = K; p.batch = 1; p.splitk = 1;
+  p.A = (const bz::bf16*)A; p.lda = K;
+  p.B = (const bz::bf16*)B; p.ldb = K;
   p.alpha = 1.0f;
   p.outf = C; p.ldc = 256;
   p.wait_limit = wait_limit;
@@ -2026,13 +2034,13 @@ static int wait_selftest(const char* name, int M, const void* A, const void* B, 
 }
 
 extern "C" int bz_gemm_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, void* stream) {
-  return wait_selftest("bz_gemm_wait_selftest", bz::tc::BM, A, B, C, wait_limit, 1, stream);
+  return wait_selftest("bz_gemm_wait_selftest", bz::tc::BM, 64, A, B, C, wait_limit, 1, stream);
 }
 
 extern "C" int bz_gemm_pair_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, int32_t withhold,
                                           void* stream) {
-  BZ_REQUIRE(withhold == 1, "bz_gemm_pair_wait_selftest: withhold %d", withhold);
-  return wait_selftest("bz_gemm_pair_wait_selftest", bz::pair::BM, A, B, C, wait_limit, withhold, stream);
+  BZ_REQUIRE(withhold >= 1 && withhold <= 3, "bz_gemm_pair_wait_selftest: withhold %d", withhold);
+  return wait_selftest("bz_gemm_pair_wait_selftest", bz::pair::BM, 192, A, B, C, wait_limit, withhold, stream);
 }
 
 extern "C" int bz_gemm_error(int32_t* value, int32_t reset) {

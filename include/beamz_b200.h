@@ -465,8 +465,10 @@ int bz_gemm_error(int32_t* value, int32_t reset);
  * major, K contiguous), C: 128 x 256 f32 (not written). Synchronizes the stream.
  * Returns BZ_ERR_TIMEOUT when the wait ran out, BZ_OK if the word stayed clear. */
 int bz_gemm_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, void* stream);
-/* The same of the CTA-pair kernel: with withhold = 1 no MMA is issued and the epilogue
- * warps of both CTAs give up on the tile. A: 256 x 64, C: 256 x 256 (not written). */
+/* The same of the CTA-pair kernel, a tile of three K slices: with withhold = 1 no MMA is
+ * issued and the epilogue warps of both CTAs give up on the tile; with 2 (3) the even (odd)
+ * CTA does not load the last slice, so the issuing thread gives up as well and the copies
+ * of the other CTA are given the time to land. A, B: 256 x 192, C: 256 x 256 (not written). */
 int bz_gemm_pair_wait_selftest(const void* A, const void* B, float* C, int32_t wait_limit, int32_t withhold,
                                void* stream);
 

@@ -79,24 +79,32 @@ def test_gemm_bounded_wait_runs_out_and_context_survives(bz):
     assert nat.gemm_error(reset=True) == 0
 
 
-def test_pair_gemm_bounded_waits_run_out_and_context_survives(bz):
-    """The CTA-pair kernel with its MMAs withheld: both CTAs' epilogue warps give up after
-    a short limit, the result is not written, and the next product is right."""
+@pytest.mark.parametrize("withhold", [1, 2, 3])
+def test_pair_gemm_bounded_waits_run_out_and_context_survives(bz, withhold):
+    """The CTA-pair kernel with its MMAs, or one CTA's last K slice, withheld: both CTAs'
+    epilogue warps give up after a short limit, the result is not written, the kernel ends
+    soon (copies in flight get milliseconds to land, not the long limit), and the
+    next product is right."""
+    import time
+
     from beamz_b200 import _native as nat
 
     st = torch.cuda.current_stream().cuda_stream
-    A = torch.randn(256, 64, device="cuda").to(torch.bfloat16)
-    B = torch.randn(256, 64, device="cuda").to(torch.bfloat16)
+    A = torch.randn(256, 192, device="cuda").to(torch.bfloat16)
+    B = torch.randn(256, 192, device="cuda").to(torch.bfloat16)
     C = torch.full((256, 256), 7.0, device="cuda")
-    for limit in (1, 2000):
-        rc = nat.gemm_pair_wait_selftest(A.data_ptr(), B.data_ptr(), C.data_ptr(), limit, 1, st)
+    for limit in (2000, 1, 1):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        rc = nat.gemm_pair_wait_selftest(A.data_ptr(), B.data_ptr(), C.data_ptr(), limit, withhold, st)
+        assert limit > 1 or time.perf_counter() - t0 < 0.5
         assert rc == nat.BZ_ERR_TIMEOUT, rc
         assert f"ran out after {limit} polls" in nat.last_error()[1]
         assert torch.all(C == 7.0)
     assert nat.gemm_error(reset=True) == 0  # the self-test cleared the word
     p = nat.Gemm()
-    p.M, p.N, p.K, p.batch, p.splitk, p.ta, p.tb = 256, 256, 64, 1, 1, 0, 1
-    p.A, p.lda, p.B, p.ldb, p.alpha, p.outf, p.ldc = A.data_ptr(), 64, B.data_ptr(), 64, 1.0, C.data_ptr(), 256
+    p.M, p.N, p.K, p.batch, p.splitk, p.ta, p.tb = 256, 256, 192, 1, 1, 0, 1
+    p.A, p.lda, p.B, p.ldb, p.alpha, p.outf, p.ldc = A.data_ptr(), 192, B.data_ptr(), 192, 1.0, C.data_ptr(), 256
     nat.gemm(p, st)
     torch.cuda.synchronize()
     want = A.float() @ B.float().T
