@@ -17,8 +17,6 @@
 // the kernel accumulates grad += -e*(E_{n+1} - E_n)/eps_r from captured forward
 // fields. The post phase then prepares the input of step n-1:
 //   e_{n-1} = mul*(dJ/dE_n + objective term), through the same source operations.
-#include <atomic>
-
 #include "bz_tile.cuh"
 
 namespace bz {
@@ -596,15 +594,9 @@ int launch_adj_tile(const bz_grid2d* g, const bz_adjoint2d* s, const bz_source_o
   constexpr int SMEM = AdjSmem<T, TS, R, NW>::BYTES;
   const auto kernel = adjoint2d_tb_kernel<T, TS, R, NW, MINB>;
   const AdjArgs<T> a = adj_args<T>(g, s, ops, phase);
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return fail(BZ_ERR_CUDA, "bz_adjoint_step2d_multi: no current device");
-  static std::atomic<unsigned long long> opted{0ull};  // devices whose limit is raised (bit per ordinal below 64)
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (!(opted.load() & bit)) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-      return fail(BZ_ERR_CUDA, "bz_adjoint_step2d_multi: cannot configure the kernel's shared memory");
-    opted.fetch_or(bit);
-  }
+  static std::atomic<unsigned long long> devices{0ull};
+  if (!raise_smem_limit((const void*)kernel, SMEM, devices))
+    return fail(BZ_ERR_CUDA, "bz_adjoint_step2d_multi: cannot configure the kernel's shared memory");
   uintptr_t bits = (uintptr_t)s->ce | (uintptr_t)s->loss;
   for (int i = 0; i < 2; ++i) bits |= (uintptr_t)s->e[i] | (uintptr_t)s->hx[i] | (uintptr_t)s->hy[i];
   const bool vec = bits % (2 * sizeof(T)) == 0;

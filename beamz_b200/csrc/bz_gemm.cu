@@ -514,12 +514,9 @@ __global__ void __launch_bounds__(tc::THREADS) gemm_tc_kernel(GemmP p) {
 }
 
 int launch_gemm_tc(const GemmP& p, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM) != cudaSuccess)
-      return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the tcgen05 kernel's shared memory");
-    configured = true;
-  }
+  static std::atomic<unsigned long long> devices{0ull};
+  if (!raise_smem_limit((const void*)gemm_tc_kernel, tc::SMEM, devices))
+    return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the tcgen05 kernel's shared memory");
   dim3 grid((unsigned)ceil_div(p.N, tc::BN), (unsigned)ceil_div(p.M, tc::BM), (unsigned)(p.batch * p.splitk));
   gemm_tc_kernel<<<grid, tc::THREADS, tc::SMEM, st>>>(p);
   return check_launch("bz_gemm_bf16");
@@ -741,12 +738,9 @@ int launch_gemm_tma(const GemmP& p, cudaStream_t st) {
   if (p.batch != 1) return 0;
   alignas(64) CUtensorMap ma, mb;
   if (!make_map(&ma, p.A, p.M, p.K, p.lda, tc::BM) || !make_map(&mb, p.B, p.N, p.K, p.ldb, tc::BN)) return 0;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tma::SMEM) != cudaSuccess)
-      return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the TMA kernel's shared memory");
-    configured = true;
-  }
+  static std::atomic<unsigned long long> devices{0ull};
+  if (!raise_smem_limit((const void*)gemm_tma_kernel, tma::SMEM, devices))
+    return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the TMA kernel's shared memory");
   dim3 grid((unsigned)ceil_div(p.N, tc::BN), (unsigned)ceil_div(p.M, tc::BM), (unsigned)p.splitk);
   gemm_tma_kernel<<<grid, tc::THREADS, tma::SMEM, st>>>(ma, mb, p);
   const int rc = check_launch("bz_gemm_bf16");
@@ -1328,7 +1322,10 @@ bool mix_eligible(const GemmP& p) {
 template <int KC, int MC, int EPI>
 int launch_mix_epi(const GemmP& p, cudaStream_t st) {
   using C = MixCfg<KC, MC>;
-  static int per_sm = 0;
+  static std::atomic<int> resident[64];  // CTAs an SM, by device ordinal
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return fail(BZ_ERR_CUDA, "bz_gemm_bf16: no current device");
+  int per_sm = dev < 64 ? resident[dev].load() : 0;
   if (per_sm == 0) {
     if (cudaFuncSetAttribute(mix_tc_kernel<KC, MC, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
             cudaSuccess ||
@@ -1338,18 +1335,18 @@ int launch_mix_epi(const GemmP& p, cudaStream_t st) {
     // resident CTAs per SM from the kernel's registers (allocated per warp in units of
     // 256), its shared memory (1 KB reserved per CTA) and the 512 TMEM columns
     cudaFuncAttributes fa;
-    int dev = 0, smem_sm = 0;
-    if (cudaFuncGetAttributes(&fa, mix_tc_kernel<KC, MC, EPI>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+    int smem_sm = 0;
+    if (cudaFuncGetAttributes(&fa, mix_tc_kernel<KC, MC, EPI>) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
       return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot query the mixing kernel's resources");
     const int regs_cta = ((fa.numRegs * 32 + 255) / 256 * 256) * (mix::THREADS / 32);
     const int by_regs = 65536 / max(1, regs_cta), by_smem = smem_sm / (C::SMEM + (int)fa.sharedSizeBytes + 1024);
     per_sm = max(1, min(min(by_regs, by_smem), min(8, 512 / (2 * C::NCOL))));
+    if (dev < 64) resident[dev].store(per_sm);
   }
   alignas(64) CUtensorMap mx;
   if (!make_map(&mx, p.B, (long long)p.batch * KC, p.N, p.ldb, KC)) return 0;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
+  int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles_n = (int)ceil_div(p.N, mix::TP);
   const long long n_tiles = (long long)p.batch * tiles_n;
@@ -1603,12 +1600,9 @@ bool wgrad_eligible(const GemmP& p) {
 template <int NC>
 int launch_wgrad_nc(const GemmP& p, cudaStream_t st) {
   constexpr int SMEM = wg::S * (wg::A_ST + NC * wg::BK * 2) + 8 * (2 * wg::S + 1) + 16 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(wgrad_tc_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-      return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the weight-gradient kernel's shared memory");
-    configured = true;
-  }
+  static std::atomic<unsigned long long> devices{0ull};
+  if (!raise_smem_limit((const void*)wgrad_tc_kernel<NC>, SMEM, devices))
+    return fail(BZ_ERR_CUDA, "bz_gemm_bf16: cannot configure the weight-gradient kernel's shared memory");
   alignas(64) CUtensorMap ma, mb;
   if (!make_map(&ma, p.A, (long long)p.batch * p.M, p.K, p.lda, p.M) ||
       !make_map(&mb, p.B, (long long)p.batch * NC, p.K, p.ldb, NC))

@@ -19,8 +19,6 @@
 //
 // After the tile is written, the block applies the source and monitor
 // operations that fall inside it, spread over all its threads.
-#include <atomic>
-
 #include "bz_tile.cuh"
 
 namespace bz {
@@ -758,15 +756,9 @@ int launch_tb(const bz_grid2d* gd, const bz_fields2d* f, const bz_source_ops* s,
   constexpr int OW = TBW - 2 * (TS + 1), OH = NW * R - 2 * TS;
   constexpr int SMEM = TbSmem<T, TS, R, NW>::BYTES;
   const auto kernel = step2d_tb_kernel<T, TS, R, NW, MINB, PWR>;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return fail(BZ_ERR_CUDA, "bz_step2d_multi: no current device");
-  static std::atomic<unsigned long long> opted{0ull};  // devices whose limit is raised (bit per ordinal below 64)
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (!(opted.load() & bit)) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-      return fail(BZ_ERR_CUDA, "bz_step2d_multi: cannot configure the kernel's shared memory");
-    opted.fetch_or(bit);
-  }
+  static std::atomic<unsigned long long> devices{0ull};
+  if (!raise_smem_limit((const void*)kernel, SMEM, devices))
+    return fail(BZ_ERR_CUDA, "bz_step2d_multi: cannot configure the kernel's shared memory");
   const Geo2D<T> g = make_geo<T>(gd);
   Ops2D<T> o = make_ops<T>(s, m);
   if (m && m->region && m->n_reg > 1) {

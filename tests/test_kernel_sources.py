@@ -37,3 +37,10 @@ def test_pair_epilogue_waits_as_one_warp():
     body = code[code.index("gemm_pair_kernel(const __grid_constant__"):]
     body = body[body.index("warp >= 2"):body.index("arrive_rank0(tempty0")]
     assert re.findall(r"\w+\(0xffffffffu, tc_wait\(tfull0", body) == ["__all_sync(0xffffffffu, tc_wait(tfull0"]
+
+
+def test_launch_settings_are_kept_per_device():
+    """What a launcher sets on a kernel holds for the device that was current, and launchers
+    run on several host threads: nothing remembers it in a plain static."""
+    for path in sorted(CSRC.glob("*.cu*")):
+        assert not re.findall(r"^\s+static (?:bool|int|unsigned|long long) .*", path.read_text(), re.M), path.name
