@@ -259,7 +259,8 @@ class AdjointFDTD2D:
         phase = 0
         grid = eng.grid
         if self._adj_block is None:
-            self._adj_block = self._time_adjoint(grid, st_, st)
+            st_.n_fwd = self.n_steps + 1 if hist else self.K + 1
+            self._adj_block = self._time_adjoint(grid, st_, torch.zeros_like(grad), st)
         if hist:  # the whole forward history is on the device: reverse steps only
             st_.fwd_step0, st_.n_fwd = 0, self.n_steps + 1
             n, tb = self.n_steps - 1, self._adj_block
@@ -294,22 +295,26 @@ class AdjointFDTD2D:
         torch.cuda.current_stream().synchronize()
         return grad.cpu().numpy() / self._adj_scale[:, None, None]
 
-    def _time_adjoint(self, grid, state, stream, reps: int = 2) -> int:
+    def _time_adjoint(self, grid, state, scratch, stream, reps: int = 2) -> int:
         """Reverse steps per launch, the fastest on this problem: blocked launches (the
         forward run's block, or a shorter one, whose gradient history is small enough for
         two blocks per SM) or single steps (a single design on a small grid leaves the
-        blocked tiles too few to fill the GPU). Timed before the backward pass, with the
-        gradient history allocated and no operations; every launch reads the still-zero
-        current copy and only adds zeros to the gradient, so nothing changes."""
+        blocked tiles too few to fill the GPU). Timed before the backward pass without the
+        operations, over the same number of steps each (up to one launch), with the planes
+        of the forward fields (``state.n_fwd`` of them) read as in the pass. Every launch reads the
+        seeded copy 0, writes copy 1, which the first reverse step overwrites, and adds to
+        ``scratch`` instead of the gradient."""
         tb = self.engine.time_block
         if tb <= 1:
             return 1
+        grad = state.grad
+        state.grad = scratch.data_ptr()
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         best = {}
         for k in sorted({tb, min(tb, 5), 1}, reverse=True):
-            n = 4 if k == 1 else 1
             t = float("inf")
-            for r in range(reps + 1):  # the first one warms up
+            for r in range(reps + 1):  # the first one, of one launch, warms up
+                n = -(-tb // k) if r > 0 else 1
                 a.record()
                 for _ in range(n):
                     nat.adjoint_step2d_multi(grid, state, None, k - 1, k, 0, stream)
@@ -318,6 +323,7 @@ class AdjointFDTD2D:
                 if r > 0:
                     t = min(t, a.elapsed_time(b) / (n * k))
             best[k] = t
+        state.grad = grad
         return min(best, key=best.get)
 
     def value_and_grad(self, eps_region):

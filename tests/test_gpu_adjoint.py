@@ -251,3 +251,42 @@ def test_reverse_tiles_match_single_steps(bz, ny, nx, pml, box, designs, precisi
     assert np.abs(grads[1]).max() > 0
     for k, g in grads.items():
         assert np.linalg.norm(g - grads[1]) <= tol * np.linalg.norm(grads[1]), k
+
+
+@pytest.mark.parametrize("history", [True, False])
+def test_reverse_block_is_timed_on_the_work_it_is_chosen_for(bz, monkeypatch, history):
+    """The launches that choose the reverse block length read the forward planes, add to
+    another buffer than the gradient, and take the same number of steps a repetition for every
+    candidate up to one launch; the pass that tunes gives the gradient of the next one."""
+    from collections import Counter
+
+    from beamz_b200.optimization import adjoint
+
+    ny, nx, dx, n = 60, 90, 20e-9, 40
+    dt = 0.99 * dx / (bz.LIGHT_SPEED * np.sqrt(2))
+    sig = np.sin(2 * np.pi * 1.9e14 * np.arange(n) * dt + 0.5)
+    src = bz.GaussianSource(position=(54 * dx, 30 * dx), width=dx, signal=sig)
+    mon = bz.Monitor(start=(60 * dx, 20 * dx), end=(60 * dx, 40 * dx))
+    p = adjoint.AdjointFDTD2D(np.full((ny, nx), 2.0), np.zeros((ny, nx)), dx, dt, n, [src], mon,
+                              np.ones(21, dtype=complex), 1.9e14, (20, 20, 20, 30), precision="fp64",
+                              checkpoint_every=20, store_history=history)
+    calls, real = [], adjoint.nat.adjoint_step2d_multi
+
+    def spy(grid, state, ops, step, k, phase, stream):
+        calls.append((ops is None, state.grad, state.n_fwd, k))
+        real(grid, state, ops, step, k, phase, stream)
+
+    monkeypatch.setattr(adjoint.nat, "adjoint_step2d_multi", spy)
+    er = 2.0 + np.random.default_rng(4).random((1, 20, 30))
+    first = p.value_and_grad(er)[1]
+    timed, run = [c for c in calls if c[0]], [c for c in calls if not c[0]]
+    assert timed and all(c[2] == (n + 1 if history else 21) for c in timed)
+    assert not {c[1] for c in timed} & {c[1] for c in run}
+    launches = Counter(c[3] for c in timed)
+    tb = max(launches)
+    reps = launches[tb] - 1  # after one launch that warms up
+    assert reps >= 2 and all(v == 1 + reps * -(-tb // k) for k, v in launches.items())
+    del calls[:]
+    second = p.value_and_grad(er)[1]
+    assert calls and not any(c[0] for c in calls) and np.abs(first).max() > 0
+    np.testing.assert_array_equal(second, first)
