@@ -434,7 +434,12 @@ __global__ void __launch_bounds__(32 * NW, MINB) step2d_tb_kernel(
   }
   // Monitors sample owned cells: the warp stages the lanes x rows that hold its points each
   // sub-step (record 10 values a pair of cells), and the block writes the points from there.
-  // A warp whose points spread over more cells than it can stage writes row by row.
+  // A warp whose points spread over more cells than it can stage (a tile crossed by eight or
+  // more adjacent lines) writes row by row: every lane searches the row's points for its two
+  // cells. (400 x 400 cells, 9 steps a launch, us a step, walking the warp's whole list for each
+  // row -> searching: 8 adjacent lines 470 -> 8.6, 64 lines 529 -> 12.3, 16 lines along y 30.8 ->
+  // 7.2; 4 lines, staged, 2.6. A map of the cells' first points in the staged cells' place takes
+  // 5.0, 6.3 and 3.3, but 64 x 64 tiles that never use it ran 3 to 14 % slower beside that code.)
   if (mk0 < mk1) {
     const int c0 = X0 + HX, c1 = min(X0 + TBW - HX, nx);
     for (int k = mk0 + lane; k < mk1; k += 32) {
@@ -660,10 +665,14 @@ __global__ void __launch_bounds__(32 * NW, MINB) step2d_tb_kernel(
           const V up = yb + i < 1 ? zero : (i > 0 ? hy[i > 0 ? i - 1 : 0] : hyu);
           const T hl = xa >= 1 ? side[i] : T(0);
           const int base = (yb + i) * nx;
-          for (int k = mk0; k < mk1; ++k) {  // every lane reads the list, the owner writes
+          int k = mk1, k1 = mk1;
+          if (own) {  // the owner writes
+            k1 = __ldg(o.mon_row + yb + i + 1);
+            k = lower_bound_i(o.mon_cell, __ldg(o.mon_row + yb + i), k1, base + xa);
+          }
+          for (; k < k1; ++k) {
             const int x = __ldg(o.mon_cell + k) - base;
-            if (x != xa && x != xa + 1) continue;
-            if (!own) continue;
+            if (x > xa + 1) break;
             const T q[9] = {lo2(ez[i]), hi2(ez[i]), lo2(hx[i]), hi2(hx[i]), lo2(hy[i]), hi2(hy[i]), lo2(up), hi2(up), hl};
             if (x == xa) write_point(q, 0, __ldg(o.mon_point + k), step, ring_slot);
             else write_point(q, 1, __ldg(o.mon_point + k), step, ring_slot);

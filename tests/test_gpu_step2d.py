@@ -226,6 +226,36 @@ def test_blocked_tiles_match_single_steps(bz, nx, ny, lossy, precision):
         assert rel_l2(dft, outs[0][1]) <= 1e-12
 
 
+@pytest.mark.parametrize("vertical", [False, True])
+def test_blocked_steps_of_dense_monitors_stay_faster_than_single_ones(bz, vertical):
+    """Sixteen adjacent lines give a tile more points than it stages. A step of a blocked
+    launch then still takes less time than a single step (they took 15 times as long when
+    every warp walked its whole list of points for each of its rows)."""
+    import torch
+
+    from beamz_b200.simulation.engine2d import Engine2D
+
+    n, dx = 400, 20e-9
+    dt = 0.99 * dx / (299792458.0 * np.sqrt(2))
+    ends = [((4, 130 + i), (n - 4, 130 + i)) for i in range(16)]
+    mons = [bz.Monitor(start=tuple(v * dx for v in (a[::-1] if vertical else a)),
+                       end=tuple(v * dx for v in (b[::-1] if vertical else b)), frequencies=[1.9e14]) for a, b in ends]
+    per_step = {}
+    for tb in (1, 7):
+        eng = Engine2D(np.full((n, n), 2.0), np.zeros((n, n)), dx, dx, dt, 200, [], mons, record=False, time_block=tb)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        launch = eng._launch_tb if tb > 1 else eng._launch
+        for _ in range(3):
+            launch(0, None)
+        a.record()
+        for _ in range(10):
+            launch(0, None)
+        b.record()
+        b.synchronize()
+        per_step[tb] = a.elapsed_time(b) / (10 * tb)
+    assert per_step[7] < per_step[1]
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 @pytest.mark.parametrize("nx,ny", [(61, 47), (150, 131), (2, 2)])
 def test_blocked_power_matches_single_steps(bz, nx, ny, precision):
