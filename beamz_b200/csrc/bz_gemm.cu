@@ -11,11 +11,12 @@
 // mma.sync.m16n8k16 (bf16 inputs, f32 accumulators). The epilogue adds an f32 (or
 // bf16) term, row/column biases, applies GELU, and stores f32 and/or bf16, or
 // accumulates atomically (batch-reduced or split-K weight gradients). Where the
-// shapes allow, bz_gemm_bf16 runs tcgen05/TMEM kernels instead: the large DFT GEMMs
-// (TMA-fed, 128 x 256 tiles), the 1x1 channel mixing (pixel-contiguous activations
-// as an MN-major TMA operand) and its weight gradients (both operands K-major,
-// reduced over pixels and designs); each is described below. The mma.sync kernel
-// remains for the shapes they do not take (the 3-channel lift layer, the pooled head).
+// shapes allow, bz_gemm_bf16 runs other kernels instead: tcgen05/TMEM ones for the large
+// DFT GEMMs (TMA-fed, 256 x 256 tiles on CTA pairs, 128 x 256 on one CTA), the 1x1 channel
+// mixing (pixel-contiguous activations as an MN-major TMA operand) and its weight
+// gradients (both operands K-major, reduced over pixels and designs), and a small
+// mma.sync one for the 3-channel lift layer; each is described below. The general kernel
+// remains for the shapes they do not take (the pooled head, the lift layer's gradients).
 #include <cuda.h>
 #include <cuda_bf16.h>
 

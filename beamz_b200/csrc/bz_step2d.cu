@@ -928,7 +928,7 @@ extern "C" int bz_step2d_multi(const bz_grid2d* g, const bz_fields2d* f, const b
   BZ_REQUIRE(tile >= 0 && tile <= 5, "bz_step2d_multi: tile must be 0..5 (got %d)", tile);
   if (n_sub == 1) return bz_step2d(g, f, s, m, step, d_step, stream);
   if (f->power != nullptr)
-    return bz::fail(BZ_ERR_UNSUPPORTED, "bz_step2d_multi: power accumulation needs bz_step2d");
+    return bz::fail(BZ_ERR_UNSUPPORTED, "bz_step2d_multi: power accumulation needs bz_step2d or bz_step2d_multi_power");
   cudaStream_t st = bz::as_stream(stream);
   return g->dtype == BZ_F32 ? bz::tb_by_steps<float>(g, f, s, m, step, n_sub, tile, d_step, st)
                             : bz::tb_by_steps<double>(g, f, s, m, step, n_sub, tile, d_step, st);

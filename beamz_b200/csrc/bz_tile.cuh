@@ -102,9 +102,12 @@ __device__ __forceinline__ void prefetch_tile(const T* const (&arr)[5], int X, i
   }
 }
 
-// Blocks between a tile and the one to prefetch: the blocks an SM runs side by side times
-// the SMs, where the arrays do not stay in L2 from one launch to the next (and there is
-// more than one such wave); 0: no prefetch.
+// Blocks between a tile and the one to prefetch, where the arrays do not stay in L2 from one
+// launch to the next (and there is more than one such distance); 0: no prefetch. The distance
+// is a wave of two blocks an SM, the large float tiles' (64 designs of 600 x 400: forward
+// launch 297 -> 288 us, 1500 reverse steps 98 -> 93 ms). Kernels of one block an SM
+// (double, power, seven and nine reverse steps) fetch two waves ahead with it, the 64 x 32
+// float tile, of three, two thirds of one; neither was tuned apart.
 inline int prefetch_distance(long long bytes, long long blocks) {
   constexpr long long WAVE = 2 * 148;
   return bytes > (100LL << 20) && blocks > 2 * WAVE ? (int)WAVE : 0;

