@@ -113,3 +113,21 @@ def test_finalising_between_steps_keeps_rows_and_times_together(bz, monkeypatch,
     np.testing.assert_allclose(np.array(mon.power_history), mag.sum(axis=1), rtol=1e-13)
     np.testing.assert_allclose(mon.power_accumulated, mag.sum(axis=0), rtol=1e-13)
     assert mon.power_accumulation_count == len(steps) and mon.last_record_step == steps[-1]
+
+
+@pytest.mark.parametrize("limit,pinned", [(2 * 3 * 3 * 8, True), (2 * 3 * 3 * 8 - 1, False)])
+def test_page_locked_memory_takes_records_up_to_its_limit(bz, monkeypatch, limit, pinned):
+    """Samples above PINNED_RECORD_BYTES a monitor reach it through pageable memory."""
+    from beamz_b200.simulation import fdtd
+
+    calls = []
+    monkeypatch.setattr(fdtd, "to_host", lambda t: calls.append(t.nbytes) or t.numpy())
+    monkeypatch.setattr(fdtd, "PINNED_RECORD_BYTES", limit)
+    sim = fdtd.FDTD.__new__(fdtd.FDTD)
+    mon = bz.Monitor(start=(0.0, 0.0), end=(0.0, 1e-6))
+    sim.monitors, sim.results, sim.accumulate_power, sim.dt = [mon], {}, False, 0.25
+    sim.engine = _RecordingEngine([mon], False)
+    sim.engine.step_index = 2
+    sim.finalize_simulation()
+    assert bool(calls) == pinned
+    np.testing.assert_array_equal(np.array(mon.fields["Hy"]), np.arange(2)[:, None] + np.arange(3) / 10.0 + 200.0)
